@@ -127,7 +127,7 @@ struct PoolDev {
   const RigidDev* rigid;        // kMaxRigid per scene
   float* wrench;                // 8 floats per sphere slot: force xyz, 0, torque xyz, 0
   float4* vel;          // grid velocity (vx, vy, vz, mass)
-  float* rec;           // per slot 16 floats: (x, y, z, m), (m v, B0), (B1..B4), (B5..B8)
+  float* rec;           // per slot 16 floats, the deposit form (see make_record): (m, q), (Bd0..3), (Bd4..7), (Bd8, xp)
   const uint32_t* slot_key;  // regroup key of each slot: (tile << 6) | cell in tile
   const SceneDev* scenes;
   uint32_t* status;     // kStatusWords per scene
@@ -163,8 +163,11 @@ __device__ __forceinline__ uint32_t item_slot(const PoolDev& p, uint32_t n32, ui
 // Grid pool index of node (ix, iy, iz) of a scene (scene-local lattice
 // coordinates), or -1 when the node lies outside the grid or, in a sparse
 // scene, in a tile without a slot.  Dense: row-major x-fastest n^3 block;
-// sparse: 64 nodes per tile slot, x-fastest inside the 4^3 tile.
-__device__ __forceinline__ int64_t node_index(const SceneDev& sc, const uint32_t* __restrict__ tile_slot, int ix,
+// sparse: 64 nodes per tile slot, x-fastest inside the 4^3 tile.  SC: the
+// scene record, or a copy of its grid fields (n, w, key_off, tile_cap,
+// grid_off).
+template <class SC>
+__device__ __forceinline__ int64_t node_index(const SC& sc, const uint32_t* __restrict__ tile_slot, int ix,
                                               int iy, int iz) {
   const int n = (int)sc.n;
   if ((unsigned)ix >= (unsigned)n || (unsigned)iy >= (unsigned)n || (unsigned)iz >= (unsigned)n) return -1;
@@ -239,6 +242,15 @@ __device__ __forceinline__ bool all_finite(const float (&v)[N]) {
 #pragma unroll
   for (int i = 0; i < N; ++i) a[i & 3] = nf_acc(a[i & 3], v[i]);
   return nf_ok((a[0] + a[1]) + (a[2] + a[3]));
+}
+
+// Lattice coordinate (x - origin) / dx of a position, each operation rounded
+// by itself: the key writers, the gather and the scatter must find the same
+// base cell floor(xp - 0.5), so the product is kept out of any contraction
+// with the subtraction that follows it (a particle within rounding of a cell
+// face would otherwise be regrouped under one cell and deposited from another).
+__device__ __forceinline__ float lattice_pos(float x, float o, float inv_dx) {
+  return __fmul_rn(__fsub_rn(x, o), inv_dx);
 }
 
 // ---------------------------------------------------------------------------
@@ -532,11 +544,13 @@ __device__ __forceinline__ void quad_weights(float fx, float* w) {
 
 // Fixed-corotated stress from a (U, s, V) decomposition of F, mpm.wgsl:532-599:
 // s_c = clamp(s, 0.1, 10), R = U V^T, J = prod s_c, hardening h by rheology,
-// P = 2 mu h (Fc - R) + lam h (J - 1) cof, S = -dt vol P Fc^T.  Returns
-// B = m C + 4/dx^2 S so that a node at offset d receives w (m v + B d).
+// P = 2 mu h (Fc - R) + lam h (J - 1) cof, S = -dt vol P Fc^T.  A node at
+// offset d (in metres) receives w (m v + B d) with B = m C + 4/dx^2 S; what is
+// returned is Bd = B dx, the change of that momentum from one node to the next
+// along each axis (the record's form, make_record).
 __device__ __forceinline__ void p2g_affine_principal(const SvdOut<double>& svd, const MatDev& md, float jp,
-                                                     float mass, float vol, const float* C, float dt, float inv_dx,
-                                                     float* B) {
+                                                     float mass, float vol, const float* C, float dt, float dx, float inv_dx,
+                                                     float* Bd) {
   // FP64-SVD form.  With Fc = U Sc V^T, R = U V^T and cof = U diag(J/sc) V^T
   // the same stress is S = -dt vol P Fc^T = -dt vol U diag(tau) U^T,
   // tau_i = 2 mu h (sc_i - 1) sc_i + lam h (J - 1) J (Kirchhoff stress in
@@ -563,23 +577,24 @@ __device__ __forceinline__ void p2g_affine_principal(const SvdOut<double>& svd, 
   float u[9];
 #pragma unroll
   for (int i = 0; i < 9; ++i) u[i] = svd.u[i];
-  const float k = -dt * vol * 4.0f * inv_dx * inv_dx;
+  const float k = -dt * vol * 4.0f * inv_dx;
+  const float mdx = mass * dx;
 #pragma unroll
   for (int c = 0; c < 3; ++c)
 #pragma unroll
     for (int r = c; r < 3; ++r) {
       const float S = k * (u[r] * tau[0] * u[c] + u[3 + r] * tau[1] * u[3 + c] + u[6 + r] * tau[2] * u[6 + c]);
-      B[3 * c + r] = mass * C[3 * c + r] + S;
-      if (r != c) B[3 * r + c] = mass * C[3 * r + c] + S;
+      Bd[3 * c + r] = mdx * C[3 * c + r] + S;
+      if (r != c) Bd[3 * r + c] = mdx * C[3 * r + c] + S;
     }
 }
 
 // Reference form (FP32 SVD); the FP64-SVD mode takes the principal form.
 template <class T>
 __device__ __forceinline__ void p2g_affine(const SvdOut<T>& svd, const MatDev& md, float jp, float mass, float vol,
-                                           const float* C, float dt, float inv_dx, float* B) {
+                                           const float* C, float dt, float dx, float inv_dx, float* Bd) {
   if constexpr (sizeof(T) == 8) {
-    p2g_affine_principal(svd, md, jp, mass, vol, C, dt, inv_dx, B);
+    p2g_affine_principal(svd, md, jp, mass, vol, C, dt, dx, inv_dx, Bd);
   } else {
     float u[9], v[9], sc[3];
 #pragma unroll
@@ -615,13 +630,14 @@ __device__ __forceinline__ void p2g_affine(const SvdOut<T>& svd, const MatDev& m
         P[3 * c + r] = k3 * (k1 * (Fc[3 * c + r] - Rcr) + k2 * cof[3 * c + r]);
       }
     // S = P Fc^T : S[c][r] = sum_k P[k][r] * Fc[k][c]
-    const float four_inv_dx2 = 4.0f * inv_dx * inv_dx;
+    const float four_inv_dx = 4.0f * inv_dx;
+    const float mdx = mass * dx;
 #pragma unroll
     for (int c = 0; c < 3; ++c)
 #pragma unroll
       for (int r = 0; r < 3; ++r) {
         const float S = P[r] * Fc[c] + P[3 + r] * Fc[3 + c] + P[6 + r] * Fc[6 + c];
-        B[3 * c + r] = mass * C[3 * c + r] + four_inv_dx2 * S;
+        Bd[3 * c + r] = mdx * C[3 * c + r] + four_inv_dx * S;
       }
   }
 }

@@ -319,7 +319,7 @@ __global__ void k_keys(PoolDev p, uint32_t n_slots) {
   uint32_t t[3], c[3];
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    const float xp = (pos[a] - o[a]) * sc.inv_dx;
+    const float xp = lattice_pos(pos[a], o[a], sc.inv_dx);
     const float bf = floorf(xp - 0.5f);
     int b = (xp == xp) ? (int)bf - win[a] : 0;
     b = b < 0 ? 0 : b;

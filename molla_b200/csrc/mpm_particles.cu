@@ -141,6 +141,10 @@ __device__ __forceinline__ uint64_t global_ns() {
 __device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(smem)), "l"(gmem) : "memory");
 }
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(smem)), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
@@ -164,6 +168,8 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
 // position planes, the F planes, mass, volume and J_p (planes PX..PZ and
 // F0..JP in plane order), then the meta word.
 constexpr int kStagedInputs = 16;
+// Lattice x of a record that deposits nothing: outside every grid.
+constexpr float kOffGrid = 1.0e30f;
 static_assert(PY == PX + 1 && PZ == PX + 2 && MASS == F0 + 9 && VOL == F0 + 10 && JP == F0 + 11,
               "the staged planes are two runs of consecutive planes");
 
@@ -220,7 +226,8 @@ __device__ __forceinline__ void particle_step(const PoolDev& p, const SceneDev& 
   SvdOut<SR> svd;
   if constexpr (kGather) {
     // ---- g2p (mpm.wgsl:1242-1353) ----
-    const float xp[3] = {(x - sc.ox) * sc.inv_dx, (y - sc.oy) * sc.inv_dx, (z - sc.oz) * sc.inv_dx};
+    const float xp[3] = {lattice_pos(x, sc.ox, sc.inv_dx), lattice_pos(y, sc.oy, sc.inv_dx),
+                         lattice_pos(z, sc.oz, sc.inv_dx)};
     const float chk[16] = {x, y, z, jp, F[0], F[1], F[2], F[3], F[4], F[5], F[6], F[7], F[8], xp[0], xp[1], xp[2]};
     if (!all_finite(chk)) {
       atomicOr(ctx.status, kFaultNumerical);
@@ -415,8 +422,8 @@ __device__ __forceinline__ void particle_step(const PoolDev& p, const SceneDev& 
 #pragma unroll
     for (int i = 0; i < 9; ++i) C[i] = plane(p, C0 + i)[s];
     bool fin = finitef(x) && finitef(y) && finitef(z) && finitef(jp) && finitef(v[0]) && finitef(v[1]) &&
-               finitef(v[2]) && finitef((x - sc.ox) * sc.inv_dx) && finitef((y - sc.oy) * sc.inv_dx) &&
-               finitef((z - sc.oz) * sc.inv_dx);
+               finitef(v[2]) && finitef(lattice_pos(x, sc.ox, sc.inv_dx)) &&
+               finitef(lattice_pos(y, sc.oy, sc.inv_dx)) && finitef(lattice_pos(z, sc.oz, sc.inv_dx));
 #pragma unroll
     for (int i = 0; i < 9; ++i) fin = fin && finitef(F[i]) && finitef(C[i]);
     if (!fin) {
@@ -424,45 +431,53 @@ __device__ __forceinline__ void particle_step(const PoolDev& p, const SceneDev& 
       ok = false;
     }
   }
-  if constexpr (kScatter) {
-    // B = m C + 4/dx^2 S for the next scatter (all-zero for a particle
-    // that faulted, which then deposits nothing).
-    float B[9];
+  if constexpr (kScatter || WRITE_KEYS) {
+    // lattice coordinates of the new position
+    const float xq[3] = {lattice_pos(x, sc.ox, sc.inv_dx), lattice_pos(y, sc.oy, sc.inv_dx),
+                         lattice_pos(z, sc.oz, sc.inv_dx)};
+    const float bf[3] = {floorf(xq[0] - 0.5f), floorf(xq[1] - 0.5f), floorf(xq[2] - 0.5f)};
+    if constexpr (kScatter) {
+      // The record in its deposit form, so that no scatter thread repeats
+      // per-particle arithmetic: Bd = B dx and, with fx = xp - base, the
+      // momentum of node (0, 0, 0), q = m v - fx0 Bdx - fx1 Bdy - fx2 Bdz
+      // (the reference's m v + B d with d = ((i, j, k) - fx) dx regrouped:
+      // node (i, j, k) receives w (m, q + i Bdx + j Bdy + k Bdz)).  A particle
+      // that faulted deposits nothing: mass 0, at a position off every grid.
+      float Bd[9];
 #pragma unroll
-    for (int i = 0; i < 9; ++i) B[i] = 0.f;
-    if (ok) {
-      if (!kGather || !reuse_svd) {
-        SR Fs[9];
+      for (int i = 0; i < 9; ++i) Bd[i] = 0.f;
+      if (ok) {
+        if (!kGather || !reuse_svd) {
+          SR Fs[9];
 #pragma unroll
-        for (int i = 0; i < 9; ++i) Fs[i] = (SR)F[i];
-        svd3<SR>(Fs, F, svd, stol, sweeps);
+          for (int i = 0; i < 9; ++i) Fs[i] = (SR)F[i];
+          svd3<SR>(Fs, F, svd, stol, sweeps);
+        }
+        p2g_affine<SR>(svd, sc.mat[mat], jp, mass, vol, C, sc.dt, sc.dx, sc.inv_dx, Bd);
       }
-      p2g_affine<SR>(svd, sc.mat[mat], jp, mass, vol, C, sc.dt, sc.inv_dx, B);
-    }
-    // Packed record (x, y, z, m), (m v, B0), (B1..B4), (B5..B8); a
-    // faulted particle gets m = 0 and deposits nothing.
-    const float mr = ok ? mass : 0.f;
-    const float vx = ok ? mass * v[0] : 0.f, vy = ok ? mass * v[1] : 0.f, vz = ok ? mass * v[2] : 0.f;
-    rec[0] = make_float4(x, y, z, mr);
-    rec[1] = make_float4(vx, vy, vz, B[0]);
-    rec[2] = make_float4(B[1], B[2], B[3], B[4]);
-    rec[3] = make_float4(B[5], B[6], B[7], B[8]);
-  }
-  if constexpr (kScatter) {
-    // sparse storage: the tiles this record's deposit will touch
-    if (sc.tile_cap && ok) {
-      const float xq[3] = {(x - sc.ox) * sc.inv_dx, (y - sc.oy) * sc.inv_dx, (z - sc.oz) * sc.inv_dx};
-      mark_stencil_tiles(sc, p.tile_mark, (int)floorf(xq[0] - 0.5f) - sc.winx, (int)floorf(xq[1] - 0.5f) - sc.winy,
-                         (int)floorf(xq[2] - 0.5f) - sc.winz);
-    }
-  }
-  if constexpr (WRITE_KEYS) {
-    const float xp[3] = {(x - sc.ox) * sc.inv_dx, (y - sc.oy) * sc.inv_dx, (z - sc.oz) * sc.inv_dx};
-    const int win[3] = {sc.winx, sc.winy, sc.winz};
-    int nbase[3];
+      const float mr = ok ? mass : 0.f;
+      float q[3];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) nbase[a] = (xp[a] == xp[a]) ? (int)floorf(xp[a] - 0.5f) - win[a] : 0;
-    p.keys_by_id[p.orig[s]] = base_key(sc, nbase);
+      for (int r = 0; r < 3; ++r) {
+        q[r] = ok ? mass * v[r] : 0.f;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) q[r] -= (ok ? xq[a] - bf[a] : 0.f) * Bd[3 * a + r];
+      }
+      rec[0] = make_float4(mr, q[0], q[1], q[2]);
+      rec[1] = make_float4(Bd[0], Bd[1], Bd[2], Bd[3]);
+      rec[2] = make_float4(Bd[4], Bd[5], Bd[6], Bd[7]);
+      rec[3] = make_float4(Bd[8], mr != 0.f ? xq[0] : kOffGrid, xq[1], xq[2]);
+      // sparse storage: the tiles this record's deposit will touch
+      if (sc.tile_cap && ok)
+        mark_stencil_tiles(sc, p.tile_mark, (int)bf[0] - sc.winx, (int)bf[1] - sc.winy, (int)bf[2] - sc.winz);
+    }
+    if constexpr (WRITE_KEYS) {
+      const int win[3] = {sc.winx, sc.winy, sc.winz};
+      int nbase[3];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) nbase[a] = (xq[a] == xq[a]) ? (int)bf[a] - win[a] : 0;
+      p.keys_by_id[p.orig[s]] = base_key(sc, nbase);
+    }
   }
 }
 
@@ -580,10 +595,10 @@ __global__ void __launch_bounds__(kGatherThreads, 5) k_g2p(PoolDev p, double tol
 }
 
 // Scatter of the next substep (mpm.wgsl:601-627): a particle with base =
-// floor(x/dx - 0.5) and fx = x/dx - base deposits, at the node of offset
-// (i,j,k), w m and w (m v + B d) with d = ((i,j,k) - fx) dx and w the
-// quadratic B-spline weight.  Particles whose record mass is zero (numerical
-// fault this substep) deposit nothing.
+// floor(xp - 0.5) deposits, at the node of offset (i,j,k), w (m, q + i Bdx +
+// j Bdy + k Bdz) with w the quadratic B-spline weight of fx = xp - base; the
+// gather writes its records in that form (particle_step).  Particles whose
+// record mass is zero (numerical fault this substep) deposit nothing.
 //
 // Persistent CTAs over items (a tile's particles from the last regrouping,
 // at most kStageMax), 192 threads.  Per item:
@@ -593,16 +608,15 @@ __global__ void __launch_bounds__(kGatherThreads, 5) k_g2p(PoolDev p, double tol
 //     The tiles use the 64-byte swizzle: 16-byte chunk k of record j sits at
 //     chunk k ^ ((j >> 1) & 3), which spreads the lanes' reads of one chunk
 //     of different records over all shared-memory banks;
-//  2. bin: every particle is binned by its current base cell among the 6^3
-//     cells whose stencils fit the tile's 8^3-node block (a counting sort in
-//     shared memory with warp-aggregated counters), so particles that moved
-//     since the regrouping are grouped with their new cell-mates; one whose
-//     stencil leaves the block deposits straight to HBM;
+//  2. bin: every particle pushes itself onto the list of its current base
+//     cell among the 6^3 cells whose stencils fit the tile's 8^3-node block,
+//     so particles that moved since the regrouping are grouped with their new
+//     cell-mates; one whose stencil leaves the block deposits straight to HBM;
 //  3. deposit: a thread takes one x-slab i of the stencil and one cell: the
 //     tile's own cells as the regrouping dealt them to warps (so that a
 //     warp's flush atomics fall on distinct banks, count-ordered within the
 //     warp), the three slabs of a cell in adjacent lanes, then the non-empty
-//     margin cells particles moved into (listed by the scan of step 2).  It
+//     margin cells particles moved into (listed by step 2).  It
 //     adds the nine slab-i node contributions of its cell's particles in
 //     registers and issues 9 x 4 shared-memory atomics for the whole cell,
 //     not per particle; no two lanes of a warp add to the same node;
@@ -611,37 +625,43 @@ __global__ void __launch_bounds__(kGatherThreads, 5) k_g2p(PoolDev p, double tol
 // Every wait on the stage is bounded (about one second); a wait that gives
 // up sets kFaultDeviceWait in the scene's status word and ends the CTA after
 // a second bounded wait for its copy in flight.
-__device__ __noinline__ void deposit_global(float4 r0, float4 r1, float4 r2, float4 r3, float4* __restrict__ acc,
+//
+// What bounds it: instruction issue and shared-memory latency, not bytes
+// (15% of DRAM rate).  Lists instead of a counting sort, records written in
+// deposit form by the gather instead of rewritten here, and the item's frame
+// in shared memory took it from 0.832 to 0.773 ms on a 16M-particle scene
+// (256^3), from 0.239 to 0.222 ms at 4M and from 43.3 to 40 us at 500k; the
+// gather pays 0.03 of its 1.26 ms for the form at 16M.
+__device__ __noinline__ void deposit_global(float4 c0, float4 c1, float4 c2, float4 c3, float4* __restrict__ acc,
                                             uint8_t* __restrict__ touched, const SceneDev* __restrict__ scp,
                                             const uint32_t* __restrict__ tile_slot) {
   const SceneDev& sc = *scp;
   const int win[3] = {sc.winx, sc.winy, sc.winz};
-  const float ox = sc.ox, oy = sc.oy, oz = sc.oz, inv_dx = sc.inv_dx, dx = sc.dx;
-  const float B[9] = {r1.w, r2.x, r2.y, r2.z, r2.w, r3.x, r3.y, r3.z, r3.w};
-  const float xp[3] = {(r0.x - ox) * inv_dx, (r0.y - oy) * inv_dx, (r0.z - oz) * inv_dx};
-  float wgt[3][3], fx[3];
+  const float Bd[9] = {c1.x, c1.y, c1.z, c1.w, c2.x, c2.y, c2.z, c2.w, c3.x};
+  const float xp[3] = {c3.y, c3.z, c3.w};
+  float wgt[3][3];
   int base[3];
   for (int a = 0; a < 3; ++a) {
     const float bf = floorf(xp[a] - 0.5f);
     base[a] = (int)bf - win[a];
-    fx[a] = xp[a] - bf;
-    quad_weights(fx[a], wgt[a]);
+    quad_weights(xp[a] - bf, wgt[a]);
   }
   for (int q = 0; q < 27; ++q) {
     const int i = q / 9, j = (q / 3) % 3, k = q % 3;
     const int64_t c = node_index(sc, tile_slot, base[0] + i, base[1] + j, base[2] + k);
     if (c < 0) continue;
     const float wt = wgt[0][i] * wgt[1][j] * wgt[2][k];
-    const float d0 = ((float)i - fx[0]) * dx, d1 = ((float)j - fx[1]) * dx, d2 = ((float)k - fx[2]) * dx;
-    const float4 v = make_float4(wt * r0.w, wt * (r1.x + B[0] * d0 + B[3] * d1 + B[6] * d2),
-                                 wt * (r1.y + B[1] * d0 + B[4] * d1 + B[7] * d2),
-                                 wt * (r1.z + B[2] * d0 + B[5] * d1 + B[8] * d2));
+    const float fi = (float)i, fj = (float)j, fk = (float)k;
+    const float4 v = make_float4(wt * c0.x, wt * (c0.y + Bd[0] * fi + Bd[3] * fj + Bd[6] * fk),
+                                 wt * (c0.z + Bd[1] * fi + Bd[4] * fj + Bd[7] * fk),
+                                 wt * (c0.w + Bd[2] * fi + Bd[5] * fj + Bd[8] * fk));
     atomicAdd(&acc[c], v);
     touch(touched, c);
   }
 }
 
 constexpr int kLocalCells = 216;  // 6^3 base cells whose stencils fit the 8^3 block
+constexpr uint32_t kListEnd = 0xffffu;
 
 // 16-byte chunk k of staged record j under the 64-byte swizzle.
 __device__ __forceinline__ float4 stage_chunk(const float4* stage, uint32_t j, uint32_t k) {
@@ -652,201 +672,150 @@ __device__ __forceinline__ void stage_store(float4* stage, uint32_t j, const flo
   for (uint32_t k = 0; k < 4; ++k) stage[4 * j + (k ^ ((j >> 1) & 3u))] = rec[k];
 }
 
-// Where an item's scatter lands: its scene's lattice and grid block, and the
-// 8^3-node block origin (rx, ry, rz) of its tile.
-struct ItemFrame {
-  float ox, oy, oz, inv_dx, dx;
-  int wx, wy, wz, rx, ry, rz, n;
+// Where an item's scatter lands, kept in shared memory so that it holds no
+// registers: the scene's grid (the fields node_index reads), the 8^3-node
+// block origin (rx, ry, rz) of its tile, and that origin with the lattice
+// window added (a record's base cell is floor(xp - 0.5) - (bx, by, bz) in the
+// block's 6^3 local cells).
+struct ScatterItem {
+  uint32_t n, w, key_off, tile_cap;
   uint64_t grid_off;
-  float4* acc;
-  uint8_t* touched;
-  const SceneDev* sc;         // the scene record (global memory)
-  const uint32_t* tile_slot;  // sparse storage: slot of every tile key
+  int rx, ry, rz, bx, by, bz;
+  uint32_t count, slot;
+  uint32_t live;  // the scene takes deposits in this launch
+  const SceneDev* sc;
+  uint32_t* status;
 };
 
-__device__ __forceinline__ ItemFrame item_frame(const SceneDev& sc, const Item& item, float4* acc, uint8_t* touched,
-                                                const uint32_t* tile_slot) {
-  ItemFrame f;
-  f.sc = &sc;
-  f.tile_slot = tile_slot;
-  f.ox = sc.ox;
-  f.oy = sc.oy;
-  f.oz = sc.oz;
-  f.inv_dx = sc.inv_dx;
-  f.dx = sc.dx;
-  f.wx = sc.winx;
-  f.wy = sc.winy;
-  f.wz = sc.winz;
-  const uint32_t w = sc.w;
+__device__ __forceinline__ void scatter_item(ScatterItem& f, const PoolDev& p, const Item& item, uint32_t slot) {
+  const SceneDev* sc = p.scenes + item.scene;
+  const uint32_t w = sc->w;
+  if (f.sc != sc) {
+    f.sc = sc;
+    f.n = sc->n;
+    f.w = w;
+    f.key_off = sc->key_off;
+    f.tile_cap = sc->tile_cap;
+    f.grid_off = sc->grid_off;
+    f.status = p.status + (size_t)sc->status * kStatusWords;
+    // A fault latched before this launch (or a spent substep budget, or a
+    // retired scene) freezes the scene; one latched by this substep's gather
+    // is handled per particle (m = 0 in its record).
+    f.live = (scene_frozen(f.status) || !sc->live) ? 0u : 1u;
+  }
   const uint32_t tx = item.tile % w, ty = (item.tile / w) % w, tz = item.tile / (w * w);
   f.rx = 4 * (int)tx - 1;
   f.ry = 4 * (int)ty - 1;
   f.rz = 4 * (int)tz - 1;
-  f.n = (int)sc.n;
-  f.grid_off = sc.grid_off;
-  f.acc = acc;
-  f.touched = touched;
-  return f;
+  f.bx = f.rx + sc->winx;
+  f.by = f.ry + sc->winy;
+  f.bz = f.rz + sc->winz;
+  f.count = item.count;
+  f.slot = slot;
 }
 
 // Shared-memory working set of one scatter item.
 struct ScatterShared {
   float acc[4][kRegionFloats];  // the 8^3-node block: m, p.x, p.y, p.z
-  uint32_t cell[kLocalCells];   // counts, then exclusive starts
-  uint16_t idx[kStageMax];      // item records sorted by local cell
+  uint32_t head[kLocalCells];   // first record of each local cell's list, or kListEnd
+  uint16_t next[kStageMax];     // next record of the same cell
   uint8_t margin[kLocalCells];  // non-empty local cells outside the tile's own 4^3
-  uint32_t total, n_margin;
+  uint32_t n_margin;
 };
 
-__device__ __forceinline__ bool core_cell_index(int lc) {
-  const int lx = lc % 6, ly = (lc / 6) % 6, lz = lc / 36;
-  return lx >= 1 && lx <= 4 && ly >= 1 && ly <= 4 && lz >= 1 && lz <= 4;
+// Scatter step 2 (bin) for a CTA of T threads: every staged record pushes
+// itself (one shared-memory exchange) onto the list of its current base cell
+// among the 6^3 local cells; the first record of a margin cell also lists the
+// cell.  One whose stencil leaves the block deposits straight to HBM.  Lists
+// take one pass and one barrier where a counting sort took a count, a scan by
+// one warp and a ranked write with a barrier after each.  The caller
+// synchronises after it.
+template <int T>
+__device__ __forceinline__ void bin_item(const float4* stage, const ScatterItem& f, const PoolDev& p, int acc_out,
+                                         ScatterShared& ss) {
+  const uint32_t count = f.count;
+  const int bx = f.bx, by = f.by, bz = f.bz;
+  for (uint32_t j = threadIdx.x; j < count; j += T) {
+    const float4 c3 = stage_chunk(stage, j, 3);
+    const int lx = (int)floorf(c3.y - 0.5f) - bx;
+    const int ly = (int)floorf(c3.z - 0.5f) - by;
+    const int lz = (int)floorf(c3.w - 0.5f) - bz;
+    if ((unsigned)lx < 6u && (unsigned)ly < 6u && (unsigned)lz < 6u) {
+      const uint32_t lc = (uint32_t)(lx + 6 * (ly + 6 * lz));
+      const uint32_t old = atomicExch(&ss.head[lc], j);
+      ss.next[j] = (uint16_t)old;
+      if (old == kListEnd && ((unsigned)(lx - 1) >= 4u || (unsigned)(ly - 1) >= 4u || (unsigned)(lz - 1) >= 4u))
+        ss.margin[atomicAdd(&ss.n_margin, 1u)] = (uint8_t)lc;
+    } else {
+      const float4 c0 = stage_chunk(stage, j, 0);
+      if (c0.x != 0.f)
+        deposit_global(c0, stage_chunk(stage, j, 1), stage_chunk(stage, j, 2), c3, p.acc[acc_out], p.touched[acc_out],
+                       f.sc, p.tile_slot);
+    }
+  }
 }
 
-// Scatter step 2 (bin) for a CTA of T threads: every staged record is binned
-// by its current base cell among the 6^3 local cells (counting sort with
-// warp-aggregated counters); one whose stencil leaves the block deposits
-// straight to HBM.  A binned record is rewritten in place in its deposit
-// form (deposit_item): with fx = x/dx - base and Bd = B dx (columns Bdx,
-// Bdy, Bdz for the x, y, z node offsets), the momentum the node of offset
-// (i, j, k) receives per unit weight is q000 + i Bdx + j Bdy + k Bdz, where
-// q000 = m v - fx0 Bdx - fx1 Bdy - fx2 Bdz (the reference's m v + B d with
-// d = ((i, j, k) - fx) dx regrouped):
-//   (m, q000), (Bdx, Bdy.x), (Bdy.y, Bdy.z, Bdz.x, Bdz.y), (Bdz.z, fx).
-// Ends with a barrier after which cell[] holds exclusive starts and idx[]
-// the sorted record indices.
-template <int T>
-__device__ __forceinline__ void bin_item(float4* stage, uint32_t count, bool live, const ItemFrame& f,
-                                         ScatterShared& ss) {
-  constexpr int kRounds = (kStageMax + T - 1) / T;
-  const uint32_t lane = threadIdx.x & 31u;
-  uint32_t bin[kRounds];  // local cell << 16 | rank, or 0xffffffff
-#pragma unroll
-  for (int q = 0; q < kRounds; ++q) {
-    const uint32_t j = threadIdx.x + q * T;
-    uint32_t lc = 0xffffu;
-    if (live && j < count) {
-      const float4 r0 = stage_chunk(stage, j, 0);
-      if (r0.w != 0.f) {
-        const float xp[3] = {(r0.x - f.ox) * f.inv_dx, (r0.y - f.oy) * f.inv_dx, (r0.z - f.oz) * f.inv_dx};
-        const float bx = floorf(xp[0] - 0.5f), by = floorf(xp[1] - 0.5f), bz = floorf(xp[2] - 0.5f);
-        const int lx = (int)bx - f.wx - f.rx;
-        const int ly = (int)by - f.wy - f.ry;
-        const int lz = (int)bz - f.wz - f.rz;
-        if ((unsigned)lx < 6u && (unsigned)ly < 6u && (unsigned)lz < 6u) {
-          lc = (uint32_t)(lx + 6 * (ly + 6 * lz));
-          const float4 r1 = stage_chunk(stage, j, 1), r2 = stage_chunk(stage, j, 2), r3 = stage_chunk(stage, j, 3);
-          const float fx0 = xp[0] - bx, fx1 = xp[1] - by, fx2 = xp[2] - bz;
-          const float dx = f.dx;
-          const float bdx[3] = {r1.w * dx, r2.x * dx, r2.y * dx};
-          const float bdy[3] = {r2.z * dx, r2.w * dx, r3.x * dx};
-          const float bdz[3] = {r3.y * dx, r3.z * dx, r3.w * dx};
-          const float q[3] = {r1.x - fx0 * bdx[0] - fx1 * bdy[0] - fx2 * bdz[0],
-                              r1.y - fx0 * bdx[1] - fx1 * bdy[1] - fx2 * bdz[1],
-                              r1.z - fx0 * bdx[2] - fx1 * bdy[2] - fx2 * bdz[2]};
-          const float4 t[4] = {make_float4(r0.w, q[0], q[1], q[2]), make_float4(bdx[0], bdx[1], bdx[2], bdy[0]),
-                               make_float4(bdy[1], bdy[2], bdz[0], bdz[1]), make_float4(bdz[2], fx0, fx1, fx2)};
-          stage_store(stage, j, t);
-        } else {
-          deposit_global(r0, stage_chunk(stage, j, 1), stage_chunk(stage, j, 2), stage_chunk(stage, j, 3), f.acc,
-                         f.touched, f.sc, f.tile_slot);
-        }
-      }
-    }
-    const uint32_t peers = __match_any_sync(0xffffffffu, lc);
-    const uint32_t leader = __ffs(peers) - 1;
-    uint32_t base = 0;
-    if (lc != 0xffffu && lane == leader) base = atomicAdd(&ss.cell[lc], (uint32_t)__popc(peers));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    bin[q] = lc == 0xffffu ? 0xffffffffu : (lc << 16) | (base + __popc(peers & ((1u << lane) - 1u)));
-  }
-  __syncthreads();
-  // exclusive scan of the 216 cell counts (warp 0, 7 cells per lane)
-  if (threadIdx.x < 32) {
-    uint32_t c[7], sum = 0;
-#pragma unroll
-    for (int k = 0; k < 7; ++k) {
-      const int cell = (int)lane * 7 + k;
-      c[k] = cell < kLocalCells ? ss.cell[cell] : 0u;
-      sum += c[k];
-    }
-    uint32_t incl = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= (uint32_t)o) incl += y;
-    }
-    uint32_t run = incl - sum;
-    uint32_t n_margin = 0;
-#pragma unroll
-    for (int k = 0; k < 7; ++k) {
-      const int cell = (int)lane * 7 + k;
-      if (cell < kLocalCells) ss.cell[cell] = run;
-      run += c[k];
-      // compact the non-empty margin cells (particles that left the tile's
-      // own cells since the regrouping) into a short list
-      const bool mar = cell < kLocalCells && c[k] != 0u && !core_cell_index(cell);
-      const uint32_t ballot = __ballot_sync(0xffffffffu, mar);
-      if (mar) ss.margin[n_margin + __popc(ballot & ((1u << lane) - 1u))] = (uint8_t)cell;
-      n_margin += __popc(ballot);
-    }
-    if (lane == 31) {
-      ss.total = incl;
-      ss.n_margin = n_margin;
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int q = 0; q < kRounds; ++q) {
-    if (bin[q] != 0xffffffffu) ss.idx[ss.cell[bin[q] >> 16] + (bin[q] & 0xffffu)] = (uint16_t)(threadIdx.x + q * T);
-  }
-  __syncthreads();
+// The tile's own cell (local cell index) and x-slab that a core thread of the
+// deposit takes, packed as lc | slab << 8: warp w holds slots 10w..10w+9 of
+// the item's table, the three slab threads of a cell in adjacent lanes (a
+// quarter-warp of a 16-byte record load then touches about three records
+// instead of eight, and the lanes that read the same record are served by one
+// broadcast); the two spare lanes of each warp (12 in all) take the 3 slabs of
+// slots 60..63.
+__device__ __forceinline__ uint32_t core_share(const uint8_t* __restrict__ order) {
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t q = warp * 2u + (lane - 30u);  // spare-lane index when lane >= 30
+  const uint32_t slot = lane < 30u ? warp * 10u + lane / 3u : 60u + q / 3u;
+  const uint32_t slab = lane < 30u ? lane % 3u : q % 3u;
+  const uint32_t c = order[slot];
+  return ((c & 3u) + 1u) + 6u * (((c >> 2) & 3u) + 1u + 6u * ((c >> 4) + 1u)) + (slab << 8);
 }
 
 // Scatter step 3 (deposit) for a CTA of T >= 192 threads.  The first 192
-// threads take the (cell, x-slab) pairs of the tile's own 64 cells: each
-// warp holds 10 cells from the per-item table `order` (k_item_order), which
-// deals the cells so that a warp's 30 flush atomics of one node and channel
-// fall on 30 different shared-memory banks, in particle-count order inside
-// the warp (scatter -18% against a plain count order); the three slab
-// threads of a cell sit in adjacent lanes (a quarter-warp of a 16-byte
-// record load then reads about three records, not eight, and lanes reading
-// the same record share a broadcast: -10%); the two spare lanes of each warp
-// take the four cells of the remaining banks.  Then all T threads share
-// the (margin cell, slab) pairs of the non-empty cells particles moved into
-// (the compact list the scan built; scanning all 152 margin cells per item
-// cost 10% of the scatter).  A thread adds the nine slab nodes of its cell's
-// particles in registers and issues 9 x 4 shared-memory atomics for the whole
-// cell; no two lanes of a warp add to the same node.
+// threads take the (cell, x-slab) pairs of the tile's own 64 cells (`share`,
+// core_share): each warp holds 10 cells from the per-item table
+// (k_item_order), which deals the cells so that a warp's 30 flush atomics of
+// one node and channel fall on 30 different shared-memory banks, in
+// particle-count order inside the warp (scatter -18% against a plain count
+// order).  Then all T threads share the (margin cell, slab) pairs of the
+// non-empty cells particles moved into.  A thread adds the nine slab nodes of
+// its cell's particles in registers and issues 9 x 4 shared-memory atomics for
+// the whole cell; no two lanes of a warp add to the same node.
 template <int T>
-__device__ __forceinline__ void deposit_item(const float4* stage, const uint8_t* __restrict__ order,
+__device__ __forceinline__ void deposit_item(const float4* stage, uint32_t share, const ScatterItem& f,
                                              ScatterShared& ss) {
   static_assert(T >= 192, "the core cells take 6 warps of 10 cells x 3 slabs");
-  const uint32_t total = ss.total;
-  // per node of the slab: (p.x, p.y) and (p.z, m), accumulated in pairs
-  float2 axy[9], azm[9];
-  // Accumulates slab `slab` of the particles of local cell lc in registers
-  // from their deposit-form records (bin_item); returns whether it had any.
-  // Node (slab, j, k) gets w_slab(fx0) w_j(fx1) w_k(fx2) (m, q000 + slab Bdx +
-  // j Bdy + k Bdz), the sums over j and k taken as running increments.
-  auto accumulate = [&](int lc, int slab) {
+  // One loop (one copy of the code) over the core pairs, then the (margin
+  // cell, slab) pairs of the non-empty margin cells.
+#pragma unroll 1
+  for (uint32_t u = threadIdx.x; u < 192u + 3u * ss.n_margin; u += T) {
+    if (u >= 192u) share = ss.margin[(u - 192u) / 3u] + (((u - 192u) % 3u) << 8);
+    uint32_t j = ss.head[share & 0xffu];
+    if (j == kListEnd) continue;
+    // Adds the particles of local cell lc in registers: node (slab, j, k) gets
+    // w_slab(fx0) w_j(fx1) w_k(fx2) (m, q + slab Bdx + j Bdy + k Bdz), the sums
+    // over j and k taken as running increments; per node of the slab (p.x, p.y)
+    // and (p.z, m), accumulated in pairs.
+    float2 axy[9], azm[9];
 #pragma unroll
     for (int q = 0; q < 9; ++q) axy[q] = azm[q] = make_float2(0.f, 0.f);
-    // the slab's B-spline weight of t = fx0 - shift: 0.5 (1.5 - fx)^2,
-    // 0.75 - (fx - 1)^2, 0.5 (fx - 0.5)^2
-    const float shift = 1.5f - 0.5f * (float)slab;
-    const bool mid = slab == 1;
-    const float fslab = (float)slab;
-    const uint32_t first = ss.cell[lc], end = lc == kLocalCells - 1 ? total : ss.cell[lc + 1];
-    for (uint32_t t = first; t < end; ++t) {
-      const uint32_t j = ss.idx[t];
+    const uint32_t lc = share & 0xffu;
+    const float fslab = (float)(share >> 8);
+    // xp - ox is the slab's argument t = fx0 - (1.5, 1, 0.5) of its weight
+    // 0.5 (1.5 - fx)^2, 0.75 - (fx - 1)^2, 0.5 (fx - 0.5)^2; xp - oy, oz are fx1, fx2
+    const float ox = (float)(f.bx + (int)(lc % 6u)) + (1.5f - 0.5f * fslab);
+    const float oy = (float)(f.by + (int)((lc / 6u) % 6u));
+    const float oz = (float)(f.bz + (int)(lc / 36u));
+#pragma unroll 1
+    do {
       const float4 c0 = stage_chunk(stage, j, 0), c1 = stage_chunk(stage, j, 1), c2 = stage_chunk(stage, j, 2),
                    c3 = stage_chunk(stage, j, 3);
-      const float ts = c3.y - shift;
-      const float wi = mid ? fmaf(-ts, ts, 0.75f) : 0.5f * ts * ts;
+      j = ss.next[j];
+      const float ts = c3.y - ox;
+      const float wi = fslab == 1.0f ? fmaf(-ts, ts, 0.75f) : 0.5f * ts * ts;
       float wy[3], wz[3];
-      quad_weights(c3.z, wy);
-      quad_weights(c3.w, wz);
+      quad_weights(c3.z - oy, wy);
+      quad_weights(c3.w - oz, wz);
       // momentum at node (slab, 0, 0), paired with the mass: (q.x, q.y), (q.z, m)
       float2 qxy = make_float2(fmaf(fslab, c1.x, c0.y), fmaf(fslab, c1.y, c0.z));
       float2 qzm = make_float2(fmaf(fslab, c1.z, c0.w), c0.x);
@@ -872,55 +841,28 @@ __device__ __forceinline__ void deposit_item(const float4* stage, const uint8_t*
           azm[3 * jj + kk] = fma2(w2, czm, azm[3 * jj + kk]);
         }
       }
-    }
-    return end > first;
-  };
-  // Adds the accumulated slab of local cell lc to the shared block.
-  auto flush = [&](int lc, int slab) {
-    const int r0 = region_index(lc % 6, (lc / 6) % 6, lc / 36) + slab;
+    } while (j != kListEnd);
+    // ... and the slab's sums to the shared block.
+    const uint32_t at = share & 0xffu;
+    const int r0 = region_index((int)(at % 6u), (int)((at / 6u) % 6u), (int)(at / 36u)) + (int)(share >> 8);
 #pragma unroll
-    for (int j = 0; j < 3; ++j)
+    for (int jj = 0; jj < 3; ++jj)
 #pragma unroll
       for (int kk = 0; kk < 3; ++kk) {
-        const int r = r0 + kRsy * j + kRsz * kk;
-        atomicAdd(&ss.acc[0][r], azm[3 * j + kk].y);
-        atomicAdd(&ss.acc[1][r], axy[3 * j + kk].x);
-        atomicAdd(&ss.acc[2][r], axy[3 * j + kk].y);
-        atomicAdd(&ss.acc[3][r], azm[3 * j + kk].x);
+        const int r = r0 + kRsy * jj + kRsz * kk;
+        atomicAdd(&ss.acc[0][r], azm[3 * jj + kk].y);
+        atomicAdd(&ss.acc[1][r], axy[3 * jj + kk].x);
+        atomicAdd(&ss.acc[2][r], axy[3 * jj + kk].y);
+        atomicAdd(&ss.acc[3][r], azm[3 * jj + kk].x);
       }
-  };
-  // local cell (in the 6^3 frame) of slot `slot` of the item's table
-  auto core_cell = [&](uint32_t slot) {
-    const uint32_t c = order[slot];
-    return (int)((c & 3u) + 1) + 6 * ((int)((c >> 2) & 3u) + 1 + 6 * ((int)(c >> 4) + 1));
-  };
-  // Warp w takes slots 10w..10w+9, the three slab threads of a cell in
-  // adjacent lanes: a quarter-warp of a 16-byte record load then touches
-  // about three records instead of eight, and the lanes that read the same
-  // record are served by one broadcast.  The two spare lanes of each warp
-  // (12 in all) take the 3 slabs of slots 60..63.
-  if (threadIdx.x < 192) {
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t q = warp * 2u + (lane - 30u);  // spare-lane index when lane >= 30
-    const uint32_t slot = lane < 30u ? warp * 10u + lane / 3u : 60u + q / 3u;
-    const int slab = (int)(lane < 30u ? lane % 3u : q % 3u);
-    const int lc = core_cell(slot);
-    if (accumulate(lc, slab)) flush(lc, slab);
-  }
-  // then the (margin cell, slab) pairs of the non-empty margin cells
-  const int n_margin = (int)ss.n_margin;
-#pragma unroll 1
-  for (int u = (int)threadIdx.x; u < 3 * n_margin; u += T) {
-    const int lc = ss.margin[u % n_margin], slab = u / n_margin;
-    if (accumulate(lc, slab)) flush(lc, slab);
   }
 }
 
 // Scatter step 4 (flush): every non-empty node of the 8^3 block goes to HBM
 // with one float4 atomic and is cleared for the next item, as are the cell
-// counters.  The caller synchronises before the block is reused.
+// lists.  The caller synchronises before the block is reused.
 template <int T>
-__device__ __forceinline__ void flush_item(const ItemFrame& f, ScatterShared& ss) {
+__device__ __forceinline__ void flush_item(const ScatterItem& f, const PoolDev& p, int acc_out, ScatterShared& ss) {
   for (int r = threadIdx.x; r < kRegionNodes; r += T) {
     const int lx = r & 7, ly = (r >> 3) & 7, lz = r >> 6;
     const int q = region_index(lx, ly, lz);
@@ -930,19 +872,21 @@ __device__ __forceinline__ void flush_item(const ItemFrame& f, ScatterShared& ss
       ss.acc[1][q] = 0.f;
       ss.acc[2][q] = 0.f;
       ss.acc[3][q] = 0.f;
-      const int64_t c = node_index(*f.sc, f.tile_slot, f.rx + lx, f.ry + ly, f.rz + lz);
+      const int64_t c = node_index(f, p.tile_slot, f.rx + lx, f.ry + ly, f.rz + lz);
       if (c >= 0) {
-        atomicAdd(&f.acc[c], make_float4(m, px, py, pz));
-        touch(f.touched, (uint64_t)c);
+        atomicAdd(&p.acc[acc_out][c], make_float4(m, px, py, pz));
+        touch(p.touched[acc_out], (uint64_t)c);
       }
     }
   }
-  for (int r = threadIdx.x; r < kLocalCells; r += T) ss.cell[r] = 0u;
+  for (int r = threadIdx.x; r < kLocalCells; r += T) ss.head[r] = kListEnd;
+  if (threadIdx.x == 0) ss.n_margin = 0;
 }
 
 __device__ __forceinline__ void clear_scatter_shared(ScatterShared& ss, int threads) {
   for (int r = threadIdx.x; r < 4 * kRegionFloats; r += threads) (&ss.acc[0][0])[r] = 0.f;
-  for (int r = threadIdx.x; r < kLocalCells; r += threads) ss.cell[r] = 0u;
+  for (int r = threadIdx.x; r < kLocalCells; r += threads) ss.head[r] = kListEnd;
+  if (threadIdx.x == 0) ss.n_margin = 0;
 }
 
 __global__ void __launch_bounds__(kScatterThreads, 4) k_p2g(PoolDev p, const __grid_constant__ CUtensorMap rec_map,
@@ -953,21 +897,16 @@ __global__ void __launch_bounds__(kScatterThreads, 4) k_p2g(PoolDev p, const __g
       reinterpret_cast<float4*>((reinterpret_cast<uintptr_t>(s_dyn) + 1023u) & ~static_cast<uintptr_t>(1023u));
   __shared__ ScatterShared ss;
   __shared__ __align__(8) uint64_t s_bar;
-  __shared__ uint32_t s_it_next;
-  float4* __restrict__ acc = p.acc[acc_out];
-  uint8_t* __restrict__ touched = p.touched[acc_out];
+  __shared__ __align__(16) Item s_desc;     // descriptor of the next item, copied ahead
+  __shared__ ScatterItem s_item[2];         // this item's frame and the next one's
+  __shared__ uint32_t s_next;
   const uint32_t n32 = p.n_items[0];
   const uint32_t n_items = n32 + p.n_items[1];
+  if (blockIdx.x >= n_items) return;
   clear_scatter_shared(ss, kScatterThreads);
-  if (threadIdx.x == 0) {
-    mbar_init(&s_bar, 1);
-    fence_mbar_init();
-  }
-  __syncthreads();
-  // Thread 0 stages item `it` (items of 1..kStageMax particles) as
-  // ceil(count / 64) tiles; rows past the item are loaded but not read.
-  auto stage = [&](uint32_t it) {
-    const Item nx = p.items[item_slot(p, n32, it)];
+  // Thread 0 stages an item (of 1..kStageMax particles) as ceil(count / 64)
+  // tiles; rows past the item are loaded but not read.
+  auto stage = [&](const Item& nx) {
     if (nx.count - 1u < (uint32_t)kStageMax) {
       const uint32_t boxes = (nx.count + kStageBoxRows - 1) / kStageBoxRows;
       fence_proxy_async_smem();
@@ -978,45 +917,55 @@ __global__ void __launch_bounds__(kScatterThreads, 4) k_p2g(PoolDev p, const __g
         tma_load_rows(s_stage + (size_t)b * kStageBoxRows * 4, &rec_map, (int)(nx.start + b * kStageBoxRows), &s_bar);
     }
   };
-  if (threadIdx.x == 0 && blockIdx.x < n_items) stage(blockIdx.x);
-  uint32_t parity = 0;
-  for (uint32_t it = blockIdx.x; it < n_items;) {
-    // this CTA's next item, taken now; its records are staged after this
-    // item's deposit
-    if (threadIdx.x == 0) s_it_next = gridDim.x + atomicAdd(p.work + 1, 1u);
-    const uint32_t slot = item_slot(p, n32, it);
+  if (threadIdx.x == 0) {
+    mbar_init(&s_bar, 1);
+    fence_mbar_init();
+    const uint32_t slot = item_slot(p, n32, blockIdx.x);
     const Item item = p.items[slot];
-    const SceneDev* __restrict__ scp = p.scenes + item.scene;
-    uint32_t* status = p.status + (size_t)scp->status * kStatusWords;
-    // A fault latched before this launch (or a spent substep budget, or a
-    // retired scene) freezes the scene; one latched by this substep's gather
-    // is handled per particle (m = 0 in its record).
-    const uint32_t fault0 = (scene_frozen(status) || !scp->live) ? 1u : 0u;
-    const ItemFrame f = item_frame(*scp, item, acc, touched, p.tile_slot);
-    const bool staged = item.count - 1u < (uint32_t)kStageMax;
-    bool ok = staged;
-    if (staged) {
-      ok = mbar_wait_bounded(&s_bar, parity);
-      parity ^= 1u;
+    stage(item);
+    s_item[0].sc = s_item[1].sc = nullptr;
+    scatter_item(s_item[0], p, item, slot);
+  }
+  __syncthreads();
+  uint32_t parity = 0;
+  for (uint32_t it = blockIdx.x; it < n_items; parity ^= 1u) {
+    const ScatterItem& f = s_item[parity];
+    // This CTA's next item, taken now; thread 0 copies its descriptor during
+    // the deposit and stages its records after it, so that no thread waits
+    // for the counter or the descriptor.
+    uint32_t next = 0;
+    if (threadIdx.x == 0) next = gridDim.x + atomicAdd(p.work + 1, 1u);
+    const uint32_t share = core_share(p.item_order + (size_t)f.slot * 64);
+    const bool staged = f.count - 1u < (uint32_t)kStageMax;
+    const bool ok = staged && mbar_wait_bounded(&s_bar, parity);
+    const bool live = ok && f.live != 0u;
+    if (live) bin_item<kScatterThreads>(s_stage, f, p, acc_out, ss);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      if (next < n_items) cp_async16(&s_desc, p.items + item_slot(p, n32, next));
+      s_next = next;
     }
-    const bool live = ok && fault0 == 0;
-    bin_item<kScatterThreads>(s_stage, item.count, live, f, ss);
-    if (live) deposit_item<kScatterThreads>(s_stage, p.item_order + (size_t)slot * 64, ss);
+    if (live) deposit_item<kScatterThreads>(s_stage, share, f, ss);
     if (__syncthreads_or(!ok)) {
       // The stage did not arrive (or the item exceeds the stage): report it,
       // wait once more (bounded) for the copy in flight and stop this CTA.
-      if (threadIdx.x == 0) atomicOr(status, kFaultDeviceWait);
-      if (staged) mbar_wait_bounded(&s_bar, parity ^ 1u);
+      if (threadIdx.x == 0) {
+        atomicOr(f.status, kFaultDeviceWait);
+        cp_async_wait_all();
+      }
+      if (staged) mbar_wait_bounded(&s_bar, parity);
       return;
     }
     // Every thread is done with the stage: the next item's copy goes now.
-    // (s_it_next was published by the bin's barriers; thread 0 overwrites
-    // it only after the barrier below.)
-    const uint32_t next = s_it_next;
-    if (threadIdx.x == 0 && next < n_items) stage(next);
-    flush_item<kScatterThreads>(f, ss);
+    it = s_next;
+    if (threadIdx.x == 0 && it < n_items) {
+      cp_async_wait_all();
+      const Item item = s_desc;
+      stage(item);
+      scatter_item(s_item[parity ^ 1u], p, item, item_slot(p, n32, it));
+    }
+    flush_item<kScatterThreads>(f, p, acc_out, ss);
     __syncthreads();
-    it = next;
   }
 }
 
@@ -1040,16 +989,15 @@ __global__ void __launch_bounds__(kFusedThreads, 2) k_g2p2g(PoolDev p, double to
   __shared__ __align__(16) SceneDev s_sc;
   __shared__ __align__(16) float4 s_vel[kRegionNodes];
   __shared__ ScatterShared ss;
-  __shared__ uint32_t s_fault;
+  __shared__ ScatterItem s_item;
   __shared__ GatherCtx s_ctx;
-  float4* __restrict__ acc = p.acc[acc_out];
-  uint8_t* __restrict__ touched = p.touched[acc_out];
   // this SVD form's range of the work list: FP32-SVD items, then FP64-SVD items
   const uint32_t n32 = p.n_items[0];
   const uint32_t it_lo = sizeof(SR) == 8 ? n32 : 0u;
   const uint32_t it_hi = sizeof(SR) == 8 ? n32 + p.n_items[1] : n32;
   const SR stol = (SR)tol;
   clear_scatter_shared(ss, kFusedThreads);
+  if (threadIdx.x == 0) s_item.sc = nullptr;
   for (uint32_t it = it_lo + blockIdx.x; it < it_hi; it += gridDim.x) {
     const uint32_t slot = item_slot(p, n32, it);
     const Item item = p.items[slot];
@@ -1058,26 +1006,27 @@ __global__ void __launch_bounds__(kFusedThreads, 2) k_g2p2g(PoolDev p, double to
       uint32_t* dst = reinterpret_cast<uint32_t*>(&s_sc);
       for (int k = threadIdx.x; k < (int)(sizeof(SceneDev) / 4); k += kFusedThreads) dst[k] = src[k];
     }
-    const SceneDev* __restrict__ scp = p.scenes + item.scene;
-    uint32_t* status = p.status + (size_t)scp->status * kStatusWords;
-    const uint32_t fault0 = (scene_frozen(status) || !scp->live) ? 1u : 0u;
-    const bool publish_vc = budget_ends(status);
-    const ItemFrame f = item_frame(*scp, item, acc, touched, p.tile_slot);
     const bool fits = item.count <= (uint32_t)kStageMax;
-    {
-      // Stage the 8^3-node velocity block (out-of-grid nodes read as zero).
-      for (int r = threadIdx.x; r < kRegionNodes; r += kFusedThreads) {
-        const int64_t c = node_index(*scp, p.tile_slot, f.rx + (r & 7), f.ry + ((r >> 3) & 7), f.rz + (r >> 6));
-        s_vel[r] = c >= 0 ? __ldg(&p.vel[c]) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-    }
     if (threadIdx.x == 0) {
-      s_fault = fault0;
-      s_ctx = GatherCtx{status, f.rx, f.ry, f.rz, publish_vc ? 1u : 0u, item.start, item.count};
-      if (!fits) atomicOr(status, kFaultDeviceWait);
+      scatter_item(s_item, p, item, slot);
+      if (!fits) {
+        s_item.live = 0u;
+        s_item.sc = nullptr;  // the flag is the item's, not the scene's
+        atomicOr(s_item.status, kFaultDeviceWait);
+      }
+      s_ctx = GatherCtx{s_item.status, s_item.rx, s_item.ry, s_item.rz, budget_ends(s_item.status) ? 1u : 0u,
+                        item.start, item.count};
     }
     __syncthreads();
-    const bool live = s_fault == 0 && fits;
+    // Stage the 8^3-node velocity block (out-of-grid nodes read as zero).
+    for (int r = threadIdx.x; r < kRegionNodes; r += kFusedThreads) {
+      const int64_t c = node_index(s_sc, p.tile_slot, s_item.rx + (r & 7), s_item.ry + ((r >> 3) & 7),
+                                   s_item.rz + (r >> 6));
+      s_vel[r] = c >= 0 ? __ldg(&p.vel[c]) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    const uint32_t share = threadIdx.x < 192 ? core_share(p.item_order + (size_t)slot * 64) : 0u;
+    __syncthreads();
+    const bool live = s_item.live != 0u;
     if (live) {
       for (uint32_t k = threadIdx.x; k < item.count; k += kFusedThreads) {
         float4 rec[4];
@@ -1087,12 +1036,13 @@ __global__ void __launch_bounds__(kFusedThreads, 2) k_g2p2g(PoolDev p, double to
                                                   reuse_svd, rec);
         stage_store(s_stage, k, rec);
       }
+      // a thread bins the records it wrote
+      bin_item<kFusedThreads>(s_stage, s_item, p, acc_out, ss);
     }
     __syncthreads();
-    bin_item<kFusedThreads>(s_stage, item.count, live, f, ss);
-    if (live) deposit_item<kFusedThreads>(s_stage, p.item_order + (size_t)slot * 64, ss);
+    if (live) deposit_item<kFusedThreads>(s_stage, share, s_item, ss);
     __syncthreads();
-    flush_item<kFusedThreads>(f, ss);
+    flush_item<kFusedThreads>(s_item, p, acc_out, ss);
     __syncthreads();
   }
 }
@@ -1122,7 +1072,6 @@ __global__ void __launch_bounds__(kScatterThreads, 2) k_p2g_det(PoolDev p, float
     const Item item = p.items[slot];
     const SceneDev* __restrict__ scp = p.scenes + item.scene;
     const uint32_t w = scp->w;
-    const float ox = scp->ox, oy = scp->oy, oz = scp->oz, inv_dx = scp->inv_dx, dx = scp->dx;
     const int winx = scp->winx, winy = scp->winy, winz = scp->winz;
     uint32_t* status = p.status + (size_t)scp->status * kStatusWords;
     const uint32_t tx = item.tile % w, ty = (item.tile / w) % w, tz = item.tile / (w * w);
@@ -1147,41 +1096,39 @@ __global__ void __launch_bounds__(kScatterThreads, 2) k_p2g_det(PoolDev p, float
       const int bx = 4 * (int)tx + cx, by = 4 * (int)ty + cy, bz = 4 * (int)tz + cz;  // this cell's base
       const int win[3] = {winx, winy, winz};
       for (uint32_t s = s_first[cell]; s < s_end[cell]; ++s) {
-        const float4 r0 = __ldg(&rec[4 * (size_t)s]);
-        if (r0.w == 0.f) continue;
-        const float4 r1 = __ldg(&rec[4 * (size_t)s + 1]);
-        const float4 r2 = __ldg(&rec[4 * (size_t)s + 2]);
-        const float4 r3 = __ldg(&rec[4 * (size_t)s + 3]);
-        const float mass = r0.w;
-        const float B[9] = {r1.w, r2.x, r2.y, r2.z, r2.w, r3.x, r3.y, r3.z, r3.w};
-        const float xp[3] = {(r0.x - ox) * inv_dx, (r0.y - oy) * inv_dx, (r0.z - oz) * inv_dx};
-        float wgt[3][3], fx[3];
+        const float4 c0 = __ldg(&rec[4 * (size_t)s]);
+        if (c0.x == 0.f) continue;
+        const float4 c1 = __ldg(&rec[4 * (size_t)s + 1]);
+        const float4 c2 = __ldg(&rec[4 * (size_t)s + 2]);
+        const float4 c3 = __ldg(&rec[4 * (size_t)s + 3]);
+        const float mass = c0.x;
+        const float xp[3] = {c3.y, c3.z, c3.w};
+        float wgt[3][3];
         int base[3];
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
           const float bf = floorf(xp[a] - 0.5f);
           base[a] = (int)bf - win[a];
-          fx[a] = xp[a] - bf;
-          quad_weights(fx[a], wgt[a]);
+          quad_weights(xp[a] - bf, wgt[a]);
         }
         const float wi = slab == 0 ? wgt[0][0] : (slab == 1 ? wgt[0][1] : wgt[0][2]);
-        const float di = ((float)slab - fx[0]) * dx;
-        const float qx[3] = {r1.x + B[0] * di, r1.y + B[1] * di, r1.z + B[2] * di};
+        const float fs = (float)slab;
+        const float qx[3] = {c0.y + fs * c1.x, c0.z + fs * c1.y, c0.w + fs * c1.z};
         const bool own = base[0] == bx && base[1] == by && base[2] == bz;
         if (!own && slab == 0 && threadIdx.x < 64) atomicOr(status, kFaultNondeterministic);
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
           const float wij = wi * wgt[1][j];
-          const float dj = ((float)j - fx[1]) * dx;
-          const float qy[3] = {qx[0] + B[3] * dj, qx[1] + B[4] * dj, qx[2] + B[5] * dj};
+          const float fj = (float)j;
+          const float qy[3] = {qx[0] + fj * c1.w, qx[1] + fj * c2.x, qx[2] + fj * c2.y};
 #pragma unroll
           for (int kk = 0; kk < 3; ++kk) {
             const float wt = wij * wgt[2][kk];
-            const float dk = ((float)kk - fx[2]) * dx;
+            const float fk = (float)kk;
             const float dm = wt * mass;
-            const float px = wt * (qy[0] + B[6] * dk);
-            const float py = wt * (qy[1] + B[7] * dk);
-            const float pz = wt * (qy[2] + B[8] * dk);
+            const float px = wt * (qy[0] + fk * c2.z);
+            const float py = wt * (qy[1] + fk * c2.w);
+            const float pz = wt * (qy[2] + fk * c3.x);
             if (own) {
               am[3 * j + kk] += dm;
               apx[3 * j + kk] += px;
