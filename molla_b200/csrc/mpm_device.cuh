@@ -18,6 +18,7 @@
 
 #include <cstdint>
 #include <cstring>
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 namespace mpm {
@@ -138,6 +139,12 @@ struct PoolDev {
   const Item* items;
   const uint32_t* n_items;
   uint32_t item_top;
+  // The gather's own cut of the same tiles: units of a few rounds of a warp,
+  // laid out as the items are (counts n_units[0], n_units[1], top unit_top).
+  const Item* units;
+  const uint32_t* n_units;
+  uint32_t unit_top;
+  const CUtensorMap* vel_maps;  // per scene slot: its dense velocity grid, in boxes of 8^3 nodes
   const uint8_t* item_order;  // per item: its tile's 64 cells by descending count at the regrouping
   // Sparse grid storage: slot of every tile key (kNoSlot: none), the tile
   // (scene-local index) of every slot of the grid pool (indexed by grid pool
@@ -145,12 +152,22 @@ struct PoolDev {
   uint32_t* tile_slot;
   uint32_t* slot_tile;
   uint8_t* tile_mark;
-  // Item counters of the persistent particle kernels (0: gather, 1:
-  // scatter), zeroed before each launch: a CTA takes its first item by its
-  // index and every later one from the counter, so the items spread over
-  // the CTAs by finishing order rather than by a fixed stride.
+  // Counters of the persistent particle kernels (kWorkGather32, ...): a warp
+  // or CTA takes its first piece of work by its index and every later one
+  // from the counter, so the work spreads by finishing order rather than by a
+  // fixed stride.  Every grid update, which precedes the gather and the
+  // scatter of a substep, zeroes them.
   uint32_t* work;
 };
+
+enum Work : int { kWorkGather32 = 0, kWorkGather64 = 1, kWorkScatter = 2, kWorkWords = 3 };
+
+// Programmatic dependent launch: the kernels of a substep are launched while
+// the one before them still runs (launch_next allows it as soon as every CTA
+// of the running kernel has started) and wait here for its results before
+// they touch anything it writes.
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __device__ __forceinline__ float* plane(const PoolDev& p, int k) { return p.planes + (size_t)k * p.cap; }
 
@@ -158,6 +175,9 @@ __device__ __forceinline__ float* plane(const PoolDev& p, int k) { return p.plan
 // items first, then the FP64-SVD items.
 __device__ __forceinline__ uint32_t item_slot(const PoolDev& p, uint32_t n32, uint32_t i) {
   return i < n32 ? i : p.item_top - 1u - (i - n32);
+}
+__device__ __forceinline__ uint32_t unit_slot(const PoolDev& p, uint32_t n32, uint32_t i) {
+  return i < n32 ? i : p.unit_top - 1u - (i - n32);
 }
 
 // Grid pool index of node (ix, iy, iz) of a scene (scene-local lattice
@@ -262,15 +282,6 @@ __device__ __forceinline__ void matmul(const T* a, const T* b, T* o) {
 #pragma unroll
     for (int r = 0; r < 3; ++r) o[3 * c + r] = a[r] * b[3 * c] + a[3 + r] * b[3 * c + 1] + a[6 + r] * b[3 * c + 2];
 }
-// u * diag(d) * v^T
-template <class T>
-__device__ __forceinline__ void sandwich(const T* u, const T* d, const T* v, T* o) {
-#pragma unroll
-  for (int c = 0; c < 3; ++c)
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-      o[3 * c + r] = (u[r] * d[0]) * v[c] + (u[3 + r] * d[1]) * v[3 + c] + (u[6 + r] * d[2]) * v[6 + c];
-}
 template <class T>
 __device__ __forceinline__ T det3(const T* a) {
   // first-column expansion; a[3*col+row]
@@ -295,20 +306,24 @@ __device__ __forceinline__ T det3(const T* a) {
 // reference's formula) is computed in FP32 with the hardware reciprocal
 // square root and division.
 //
-// The FP32 form accumulates V in FP32; sigma_i = |F v_i| and u_i = F v_i /
-// sigma_i in FP32.
+// V accumulates in FP32 in both forms and U is held in FP32 (its consumers,
+// the stress record and F's update, are FP32); sigma carries the form's
+// precision.
 //
-// The FP64 form (svd3<double>) is mixed precision: V accumulates the same
-// rotations in FP64 with c = (1 + t^2)^(-1/2) Newton-refined to FP64 and
-// s = t c, so V stays orthogonal to FP64 rounding.  sigma_i = |F v_i| and
-// u_i = F v_i / sigma_i are FP64.  Double division and square roots are replaced by
-// Newton-Raphson refinement of single-precision seeds (two steps each,
-// quadratic convergence from 2^-22 to below 2^-52).
-// U is held in FP32 in both forms: its consumers (the stress record and
-// the rebuilt F) are FP32, while sigma and V carry the form's precision.
+// FP32 form: sigma_i = |F v_i| and u_i = F v_i / sigma_i in FP32 (hardware
+// reciprocal square root and one Newton step), and e_i = sigma_i - 1 from the
+// eigenvalue of A' where F is near a rotation: lambda'_i = sigma_i^2 - 1, so
+// e_i = lambda'_i / (1 + sigma_i) keeps the relative precision of A' where
+// sigma_i - 1 would keep only the half ulp of 1 that sigma_i was rounded to.
+//
+// FP64 form (svd3<double>): sigma_i = |F v_i| / |v_i| in FP64.  Double
+// division and square roots are replaced by Newton-Raphson refinement of
+// single-precision seeds (two steps each, quadratic convergence from 2^-22 to
+// below 2^-52).
 template <class T> struct SvdOut {
   float u[9], v[9];
   T s[3];
+  float e[3];  // sigma - 1 (FP32 form only)
 };
 
 // Newton-Raphson reciprocal square root of x > 0: y <- y (3 - x y^2) / 2
@@ -416,6 +431,7 @@ __device__ __forceinline__ void svd3(const T* f, const float* f32, SvdOut<T>& o,
 #pragma unroll
   for (int i = 0; i < 9; ++i) v[i] = (i % 4 == 0) ? 1.0f : 0.0f;
   const float ftol = (float)tol;
+#pragma unroll 1
   for (int sweep = 0; sweep < max_sweeps; ++sweep) {
     float max_off = 0.0f;
     jacobi_rot<0, 1>(a, v, ftol, max_off);
@@ -430,18 +446,17 @@ __device__ __forceinline__ void svd3(const T* f, const float* f32, SvdOut<T>& o,
       const float y = f[1] * v[3 * i] + f[4] * v[3 * i + 1] + f[7] * v[3 * i + 2];
       const float z = f[2] * v[3 * i] + f[5] * v[3 * i + 1] + f[8] * v[3 * i + 2];
       const float q = x * x + y * y + z * z;
-      const float s = sqrtf(q);  // correctly rounded: the stress depends on s - 1
-      o.s[i] = s;
-      if (s > 1.0e-12f) {
-        const float inv = __frcp_rn(s);
-        o.u[3 * i] = x * inv;
-        o.u[3 * i + 1] = y * inv;
-        o.u[3 * i + 2] = z * inv;
-      } else {
-        o.u[3 * i] = i == 0 ? 1.0f : 0.0f;
-        o.u[3 * i + 1] = i == 1 ? 1.0f : 0.0f;
-        o.u[3 * i + 2] = i == 2 ? 1.0f : 0.0f;
-      }
+      // sqrt(q) and its reciprocal by one Newton step each; q = NaN or
+      // infinite gives NaN, which the caller's check of sigma finds
+      const float r = rsqrtf(q);
+      float s = q * r;
+      s = fmaf(fmaf(-s, s, q), 0.5f * r, s);
+      const bool zero = q <= 1.0e-24f;
+      o.s[i] = zero ? 0.0f : s;
+      const float inv = r * fmaf(-0.5f * q * r, r, 1.5f);
+      o.u[3 * i] = zero ? (i == 0 ? 1.0f : 0.0f) : x * inv;
+      o.u[3 * i + 1] = zero ? (i == 1 ? 1.0f : 0.0f) : y * inv;
+      o.u[3 * i + 2] = zero ? (i == 2 ? 1.0f : 0.0f) : z * inv;
     } else {
       // sigma_i = |F v_i| / |v_i| in FP64: a Rayleigh quotient, second order
       // in the direction error of the FP32 v_i, with the norm of v_i (1 up
@@ -504,6 +519,10 @@ __device__ __forceinline__ void svd3(const T* f, const float* f32, SvdOut<T>& o,
         o.s[i] *= (T)sg;
       }
     }
+    const float top = fmaxf(fmaxf(fabsf(a[0][0]), fabsf(a[1][1])), fabsf(a[2][2]));
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+      o.e[i] = top < 0.25f && o.s[i] > 0.5f ? __fdividef(a[i][i], 1.0f + (float)o.s[i]) : (float)o.s[i] - 1.0f;
   }
 }
 
@@ -544,39 +563,46 @@ __device__ __forceinline__ void quad_weights(float fx, float* w) {
 
 // Fixed-corotated stress from a (U, s, V) decomposition of F, mpm.wgsl:532-599:
 // s_c = clamp(s, 0.1, 10), R = U V^T, J = prod s_c, hardening h by rheology,
-// P = 2 mu h (Fc - R) + lam h (J - 1) cof, S = -dt vol P Fc^T.  A node at
-// offset d (in metres) receives w (m v + B d) with B = m C + 4/dx^2 S; what is
-// returned is Bd = B dx, the change of that momentum from one node to the next
-// along each axis (the record's form, make_record).
-__device__ __forceinline__ void p2g_affine_principal(const SvdOut<double>& svd, const MatDev& md, float jp,
-                                                     float mass, float vol, const float* C, float dt, float dx, float inv_dx,
-                                                     float* Bd) {
-  // FP64-SVD form.  With Fc = U Sc V^T, R = U V^T and cof = U diag(J/sc) V^T
-  // the same stress is S = -dt vol P Fc^T = -dt vol U diag(tau) U^T,
-  // tau_i = 2 mu h (sc_i - 1) sc_i + lam h (J - 1) J (Kirchhoff stress in
-  // the principal frame).  sc_i - 1 and J - 1 are formed in FP64, so the
-  // small-strain stress keeps full FP32 relative precision instead of
-  // cancelling in Fc - R.
-  double scd[3];
+// P = 2 mu h (Fc - R) + lam h (J - 1) cof, S = -dt vol P Fc^T.  With Fc = U Sc
+// V^T and cof = U diag(J/sc) V^T that is S = -dt vol U diag(tau) U^T, tau_i = 2
+// mu h (sc_i - 1) sc_i + lam h (J - 1) J (the Kirchhoff stress in the principal
+// frame): a quarter of the arithmetic, and sc_i - 1 and J - 1, formed in FP64
+// or from the FP32 form's e, keep their relative precision at small strain
+// where Fc - R cancels.  A node at offset d (in metres) receives w (m v + B d)
+// with B = m C + 4/dx^2 S; what is returned is Bd = B dx, the change of that
+// momentum from one node to the next along each axis (the record's form).
+template <class T>
+__device__ __forceinline__ void p2g_affine(const SvdOut<T>& svd, const MatDev& md, float jp, float mass, float vol,
+                                           const float* C, float dt, float dx, float inv_dx, float* Bd) {
+  float sc[3], e[3], J, jm1;
+  if constexpr (sizeof(T) == 8) {
+    double scd[3];
 #pragma unroll
-  for (int i = 0; i < 3; ++i) scd[i] = fmin(fmax(svd.s[i], 0.1), 10.0);
-  const double Jd = scd[0] * scd[1] * scd[2];
-  const float J = (float)Jd;
-  const float jm1 = (float)(Jd - 1.0);
-  float h = 1.0f;
-  if (md.rheo == 1) {
-    h = expf(clampf(-md.hardening * jp, -3.0f, 3.0f));
-  } else if (md.rheo == 0) {
-    h = expf(clampf(jp, -3.0f, 3.0f));
+    for (int i = 0; i < 3; ++i) {
+      scd[i] = fmin(fmax(svd.s[i], 0.1), 10.0);
+      sc[i] = (float)scd[i];
+      e[i] = (float)(scd[i] - 1.0);
+    }
+    const double Jd = scd[0] * scd[1] * scd[2];
+    J = (float)Jd;
+    jm1 = (float)(Jd - 1.0);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      sc[i] = clampf(svd.s[i], 0.1f, 10.0f);
+      e[i] = sc[i] == svd.s[i] ? svd.e[i] : sc[i] - 1.0f;
+    }
+    const float e01 = e[0] + e[1] + e[0] * e[1];
+    jm1 = e01 + e[2] + e01 * e[2];
+    J = sc[0] * sc[1] * sc[2];
   }
+  const float h = md.rheo == 2 ? 1.0f : expf(clampf(md.rheo == 1 ? -md.hardening * jp : jp, -3.0f, 3.0f));
   const float k1 = 2.0f * md.mu * h;
   const float kv = md.lam * h * jm1 * J;
   float tau[3];
 #pragma unroll
-  for (int i = 0; i < 3; ++i) tau[i] = k1 * (float)(scd[i] - 1.0) * (float)scd[i] + kv;
-  float u[9];
-#pragma unroll
-  for (int i = 0; i < 9; ++i) u[i] = svd.u[i];
+  for (int i = 0; i < 3; ++i) tau[i] = k1 * e[i] * sc[i] + kv;
+  const float* u = svd.u;
   const float k = -dt * vol * 4.0f * inv_dx;
   const float mdx = mass * dx;
 #pragma unroll
@@ -589,76 +615,15 @@ __device__ __forceinline__ void p2g_affine_principal(const SvdOut<double>& svd, 
     }
 }
 
-// Reference form (FP32 SVD); the FP64-SVD mode takes the principal form.
-template <class T>
-__device__ __forceinline__ void p2g_affine(const SvdOut<T>& svd, const MatDev& md, float jp, float mass, float vol,
-                                           const float* C, float dt, float dx, float inv_dx, float* Bd) {
-  if constexpr (sizeof(T) == 8) {
-    p2g_affine_principal(svd, md, jp, mass, vol, C, dt, dx, inv_dx, Bd);
-  } else {
-    float u[9], v[9], sc[3];
-#pragma unroll
-    for (int i = 0; i < 9; ++i) {
-      u[i] = svd.u[i];
-      v[i] = (float)svd.v[i];
-    }
-#pragma unroll
-    for (int i = 0; i < 3; ++i) sc[i] = clampf((float)svd.s[i], 0.1f, 10.0f);
-    float h = 1.0f;
-    if (md.rheo == 1) {
-      h = expf(clampf(-md.hardening * jp, -3.0f, 3.0f));
-    } else if (md.rheo == 0) {
-      h = expf(clampf(jp, -3.0f, 3.0f));
-    }
-    const float mu_h = md.mu * h;
-    const float lam_h = md.lam * h;
-    const float J = sc[0] * sc[1] * sc[2];
-    const float cofd[3] = {sc[1] * sc[2], sc[0] * sc[2], sc[0] * sc[1]};
-    float Fc[9], cof[9];
-    sandwich(u, sc, v, Fc);
-    sandwich(u, cofd, v, cof);
-    const float k1 = 2.0f * mu_h;
-    const float k2 = lam_h * (J - 1.0f);
-    const float k3 = -dt * vol;
-    float P[9];
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-#pragma unroll
-      for (int r = 0; r < 3; ++r) {
-        // R = U V^T
-        const float Rcr = u[r] * v[c] + u[3 + r] * v[3 + c] + u[6 + r] * v[6 + c];
-        P[3 * c + r] = k3 * (k1 * (Fc[3 * c + r] - Rcr) + k2 * cof[3 * c + r]);
-      }
-    // S = P Fc^T : S[c][r] = sum_k P[k][r] * Fc[k][c]
-    const float four_inv_dx = 4.0f * inv_dx;
-    const float mdx = mass * dx;
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-#pragma unroll
-      for (int r = 0; r < 3; ++r) {
-        const float S = P[r] * Fc[c] + P[3 + r] * Fc[3 + c] + P[6 + r] * Fc[6 + c];
-        Bd[3 * c + r] = mdx * C[3 * c + r] + four_inv_dx * S;
-      }
-  }
-}
-
 // Plasticity return mapping on (U, s, V), mpm.wgsl:1366-1479.  Writes the
 // projected, safety-clamped singular values into s (in place), updates jp.
 // Returns false on a numerical fault.
 template <class T>
 __device__ __forceinline__ bool plasticity_project(SvdOut<T>& svd, const MatDev& md, float& jp, bool& changed) {
+  // Finite singular values imply finite U and V: sigma_i = |F v_i| and u_i = F
+  // v_i / sigma_i, and a NaN in V or an overflow reaches sigma.
   float s[3] = {(float)svd.s[0], (float)svd.s[1], (float)svd.s[2]};
-  {
-    float chk[21];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) chk[a] = s[a];
-#pragma unroll
-    for (int i = 0; i < 9; ++i) {
-      chk[3 + 2 * i] = svd.u[i];
-      chk[4 + 2 * i] = svd.v[i];
-    }
-    if (!all_finite(chk)) return false;
-  }
+  if (!all_finite(s)) return false;
   T ns[3] = {svd.s[0], svd.s[1], svd.s[2]};
   float dq = 0.0f;
   bool jp_replace = false;
@@ -719,8 +684,11 @@ __device__ __forceinline__ bool plasticity_project(SvdOut<T>& svd, const MatDev&
     T x = ns[a];
     x = x < T(0.05) ? T(0.05) : x;
     x = x > T(20) ? T(20) : x;
-    changed = changed || x != svd.s[a];
-    svd.s[a] = x;
+    if (x != svd.s[a]) {
+      changed = true;
+      svd.s[a] = x;
+      if constexpr (sizeof(T) == 4) svd.e[a] = x - 1.0f;
+    }
   }
   jp = jp_replace ? jp_new : clampf(jp + dq, 0.0f, 5.0f);
   return true;

@@ -132,6 +132,9 @@ __global__ void __launch_bounds__(kCellThreads, 5) k_grid_update(PoolDev p, cons
                                                               uint64_t total_cells, int acc_in, int count_substep) {
   static_assert(kCellThreads == kCellBlock, "one thread per cell of a grid-pool block");
   constexpr int K = kGridBlocksPerCta;
+  launch_next();
+  wait_previous();
+  if (blockIdx.x == 0 && threadIdx.x < (unsigned)kWorkWords) p.work[threadIdx.x] = 0u;
   // Every load of the marks and of the accumulators is issued before any is
   // used, so that a thread keeps K requests in flight.
   uint32_t sid[K];
@@ -421,10 +424,13 @@ __global__ void k_tile_start(const uint32_t* __restrict__ sorted_keys, uint32_t 
 // range of the key space).  Items of FP32-SVD scenes take slots from 0 up
 // (count n_items[0]), items of FP64-SVD scenes slots from item_top - 1 down
 // (count n_items[1]), so that the gather of each SVD form is one launch over
-// a contiguous range.
+// a contiguous range.  The gather's units are cut from the same tiles in the
+// same way (counts n_items[2], n_items[3]), into equal pieces of whole rounds
+// of a warp and at most about `unit` slots.
 __global__ void k_items(const uint32_t* __restrict__ tile_start, uint32_t K, const uint32_t* __restrict__ key_scene,
                         const SceneDev* __restrict__ scenes, uint32_t chunk, uint32_t item_top,
-                        Item* __restrict__ items, uint32_t* __restrict__ n_items, uint32_t* __restrict__ tile_item) {
+                        Item* __restrict__ items, uint32_t unit, uint32_t unit_top, Item* __restrict__ units,
+                        uint32_t* __restrict__ n_items, uint32_t* __restrict__ tile_item) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= K) return;
   const uint32_t a = tile_start[t], b = tile_start[t + 1];
@@ -432,19 +438,25 @@ __global__ void k_items(const uint32_t* __restrict__ tile_start, uint32_t K, con
   const uint32_t scene = key_scene[t];
   if (scene == 0xffffffffu) return;  // no live scene holds this key (cannot carry particles)
   const uint32_t cnt = b - a;
-  chunk = chunk ? chunk : cnt;
-  const uint32_t pieces = (cnt + chunk - 1) / chunk;
+  const uint32_t tile = t - scenes[scene].key_off;
   const bool up = scenes[scene].svd64 == 0u;
-  const uint32_t base = atomicAdd(&n_items[up ? 0 : 1], pieces);
-  for (uint32_t i = 0; i < pieces; ++i) {
-    Item it;
-    it.start = a + i * chunk;
-    it.count = min(chunk, cnt - i * chunk);
-    it.scene = scene;
-    it.tile = t - scenes[scene].key_off;
-    const uint32_t slot = up ? base + i : item_top - 1u - (base + i);
-    items[slot] = it;
-    if (tile_item && i == 0) tile_item[t] = slot;
+  {
+    chunk = chunk ? chunk : cnt;
+    const uint32_t pieces = (cnt + chunk - 1) / chunk;
+    const uint32_t base = atomicAdd(&n_items[up ? 0 : 1], pieces);
+    for (uint32_t i = 0; i < pieces; ++i) {
+      const uint32_t slot = up ? base + i : item_top - 1u - (base + i);
+      items[slot] = Item{a + i * chunk, min(chunk, cnt - i * chunk), scene, tile};
+      if (tile_item && i == 0) tile_item[t] = slot;
+    }
+  }
+  {
+    const uint32_t want = (cnt + unit - 1) / unit;
+    const uint32_t part = ((cnt + want - 1) / want + 31u) & ~31u;
+    const uint32_t pieces = (cnt + part - 1) / part;
+    const uint32_t base = atomicAdd(&n_items[up ? 2 : 3], pieces);
+    for (uint32_t i = 0; i < pieces; ++i)
+      units[up ? base + i : unit_top - 1u - (base + i)] = Item{a + i * part, min(part, cnt - i * part), scene, tile};
   }
 }
 
@@ -622,8 +634,8 @@ cudaError_t launch_grid_update(const PoolDev& p, const uint32_t* block_scene, ui
   const uint64_t pool_blocks = (total_cells + kCellThreads - 1) / kCellThreads;
   const uint64_t blocks = (pool_blocks + kGridBlocksPerCta - 1) / kGridBlocksPerCta;
   if (blocks == 0) return cudaSuccess;
-  k_grid_update<<<(unsigned)blocks, kCellThreads, 0, st>>>(p, block_scene, total_cells, acc_in, count_substep);
-  return cudaGetLastError();
+  return launch_dependent(k_grid_update, (int)blocks, kCellThreads, 0, st, p, block_scene, total_cells, acc_in,
+                          count_substep);
 }
 
 cudaError_t launch_grid_jacobi(const PoolDev& p, const uint32_t* block_scene, uint64_t total_cells, int acc_in,
@@ -691,13 +703,14 @@ cudaError_t launch_reorder(const float* src, float* dst, uint32_t cap, const uin
 
 cudaError_t launch_items(const uint32_t* sorted_keys, int shift, uint32_t n_live, uint32_t K, uint32_t* tile_start,
                          const uint32_t* key_scene, const SceneDev* scenes, uint32_t chunk, uint32_t item_top,
-                         Item* items, uint32_t* n_items, uint32_t* tile_item, cudaStream_t st) {
-  cudaMemsetAsync(n_items, 0, 2 * sizeof(uint32_t), st);
+                         Item* items, uint32_t unit, uint32_t unit_top, Item* units, uint32_t* n_items,
+                         uint32_t* tile_item, cudaStream_t st) {
+  cudaMemsetAsync(n_items, 0, 4 * sizeof(uint32_t), st);
   if (tile_item) cudaMemsetAsync(tile_item, 0xff, (size_t)(K + 1) * sizeof(uint32_t), st);
   k_tile_start<<<(K + 1 + 255) / 256, 256, 0, st>>>(sorted_keys, n_live, K, shift, tile_start);
   if (K > 0)
-    k_items<<<(K + 255) / 256, 256, 0, st>>>(tile_start, K, key_scene, scenes, chunk, item_top, items, n_items,
-                                             tile_item);
+    k_items<<<(K + 255) / 256, 256, 0, st>>>(tile_start, K, key_scene, scenes, chunk, item_top, items, unit, unit_top,
+                                             units, n_items, tile_item);
   return cudaGetLastError();
 }
 

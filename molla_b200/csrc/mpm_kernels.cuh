@@ -16,12 +16,32 @@ constexpr int kScatterThreads = 192;  // 64 cells x 3 x-slabs of one tile
 constexpr int kFusedThreads = 256;    // fused gather + scatter: 2 CTAs per SM (128 registers per thread)
 constexpr uint32_t kCellBlock = 256;  // grid pool granularity: one scene per 256-cell block
 
+// Launches a kernel that calls wait_previous() as a programmatic dependent of
+// the stream's last kernel: its CTAs are scheduled as that kernel's leave, and
+// its set-up overlaps that kernel's tail (a 5 us kernel after a 20 us one cost
+// about 2 us of gap without it).
+template <class... P, class... A>
+inline cudaError_t launch_dependent(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t st,
+                                    A... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, (P)args...);
+}
+
 enum GatherMode : int { kRecord = 0, kG2P = 1, kG2PRecord = 2 };
 
 // publish_all: the gather writes v and C for every particle (a call's last
 // substep), not only for scenes whose substep budget ends.
 cudaError_t launch_gather(int mode, bool write_keys, bool svd_fp64, const PoolDev& p, double tol, int sweeps,
-                          int reuse, int grid, cudaStream_t st, bool publish_all = false);
+                          int grid, cudaStream_t st, bool publish_all = false);
 // The scatter stages its records with TMA through `rec_map`, a 2-D tensor
 // map of the record buffer (16 floats x cap, 64-byte swizzle) built by
 // make_record_map.
@@ -30,6 +50,9 @@ cudaError_t launch_scatter(const PoolDev& p, const CUtensorMap& rec_map, int acc
 // completes and reports kFaultDeviceWait: the scatter's timeout path.
 cudaError_t launch_selftest_wait(uint32_t* status, unsigned long long* waited_ns, cudaStream_t st);
 bool make_record_map(CUtensorMap* out, const float* rec, uint32_t cap, std::string* err);
+// 3-D tensor map of a dense scene's n^3 velocity grid in boxes of 8^3 nodes,
+// from which the gather stages a tile's velocity block (n >= 8).
+bool make_velocity_map(CUtensorMap* out, const float4* vel, uint32_t n, std::string* err);
 // Deterministic (fixed-order) scatter: per-tile blocks, then a combine pass.
 cudaError_t launch_scatter_det(const PoolDev& p, float4* blocks, int acc_out, int grid, cudaStream_t st);
 cudaError_t launch_combine_det(const PoolDev& p, const float4* blocks, const uint32_t* tile_item, uint32_t max_items,
@@ -46,7 +69,7 @@ constexpr int kStageBoxRows = 64;                // records per TMA box of the s
 int gather_grid_size(bool svd_fp64);
 // Fused gather + scatter of a non-final substep (k_g2p2g): gather with the B
 // record kept in shared memory, then the record deposit into acc[acc_out].
-cudaError_t launch_fused(bool write_keys, bool svd_fp64, const PoolDev& p, double tol, int sweeps, int reuse,
+cudaError_t launch_fused(bool write_keys, bool svd_fp64, const PoolDev& p, double tol, int sweeps,
                          int acc_out, int grid, cudaStream_t st);
 int fused_grid_size(bool svd_fp64);
 int scatter_grid_size();
@@ -80,7 +103,8 @@ cudaError_t launch_vel_copy(const uint8_t* touched, const uint32_t* block_scene,
 // [0, n_items[0]), FP64-SVD items in [item_top - n_items[1], item_top).
 cudaError_t launch_items(const uint32_t* sorted_keys, int shift, uint32_t n_live, uint32_t K, uint32_t* tile_start,
                          const uint32_t* key_scene, const SceneDev* scenes, uint32_t chunk, uint32_t item_top,
-                         Item* items, uint32_t* n_items, uint32_t* tile_item, cudaStream_t st);
+                         Item* items, uint32_t unit, uint32_t unit_top, Item* units, uint32_t* n_items,
+                         uint32_t* tile_item, cudaStream_t st);
 // Rebuilds the tile maps of the sparse scenes from the tiles the last gather
 // marked (two launches).
 cudaError_t launch_tiles_finalize(const PoolDev& p, const uint32_t* key_scene, uint32_t K, uint32_t n_scenes,

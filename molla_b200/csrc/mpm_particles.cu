@@ -37,11 +37,6 @@ namespace mpm {
 
 namespace {
 
-struct SharedGather {
-  float4 vel[kRegionNodes];
-  float fallback[kGatherThreads][13];  // per-thread result slot of gather_global
-};
-
 __device__ __forceinline__ int region_index(int lx, int ly, int lz) { return lx + kRsy * ly + kRsz * lz; }
 
 // Regroup key of a particle from its base cell: ((scene tile offset + tile)
@@ -64,8 +59,7 @@ __device__ __forceinline__ uint32_t base_key(const SceneDev& sc, const int* base
 // (it left its tile since the last regrouping): 27 global reads with the
 // reference's out-of-grid skip.  Kept out of line and rolled so that the
 // unrolled shared-memory path stays small; it takes scalars and writes
-// v (3) and G = sum w gv d^T (9) to the caller's shared-memory slot, so the
-// call needs no local memory.
+// v (3) and G = sum w gv d^T (9) to out.
 __device__ __noinline__ void gather_global(const float4* __restrict__ vel_pool, const SceneDev& sc,
                                            const uint32_t* __restrict__ tile_slot, float xp0, float xp1, float xp2,
                                            float* out) {
@@ -83,6 +77,7 @@ __device__ __noinline__ void gather_global(const float4* __restrict__ vel_pool, 
   }
   float acc[12];
   for (int i = 0; i < 12; ++i) acc[i] = 0.f;
+#pragma unroll 1
   for (int q = 0; q < 27; ++q) {
     const int i = q / 9, j = (q / 3) % 3, k = q % 3;
     const int64_t c = node_index(sc, tile_slot, base[0] + i, base[1] + j, base[2] + k);
@@ -122,6 +117,21 @@ __device__ __forceinline__ void tma_load_rows(void* dst, const CUtensorMap* map,
       "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(row), "r"(smem_addr(bar))
       : "memory");
 }
+// 3-D TMA box (32 floats x 8 x 8: the 8^3 nodes of a velocity block) from
+// coordinates (x, y, z); x is a multiple of four floats.
+__device__ __forceinline__ void tma_load_box(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::
+          "r"(smem_addr(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_addr(bar))
+      : "memory");
+}
+// Makes a tensor map in global memory, written by an earlier copy, visible to
+// the TMA loads of this thread.
+__device__ __forceinline__ void fence_tensormap(const CUtensorMap* map) {
+  asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(reinterpret_cast<uint64_t>(map))
+               : "memory");
+}
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t done;
   asm volatile(
@@ -136,8 +146,8 @@ __device__ __forceinline__ uint64_t global_ns() {
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
-// Ampere-style asynchronous 4-byte global -> shared copies (cp.async), in
-// commit groups; a thread waits for its own groups.
+// Ampere-style asynchronous global -> shared copies (cp.async) of 4 or 16
+// bytes; a thread waits for its own.
 __device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(smem)), "l"(gmem) : "memory");
 }
@@ -145,11 +155,6 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(smem)), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
 
 // Waits for the phase of `bar` with the given parity to complete; gives up
 // (returns false) after about one second.
@@ -168,15 +173,31 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
 // position planes, the F planes, mass, volume and J_p (planes PX..PZ and
 // F0..JP in plane order), then the meta word.
 constexpr int kStagedInputs = 16;
+static_assert(PY == PX + 1 && PZ == PX + 2 && MASS == F0 + 9 && VOL == F0 + 10 && JP == F0 + 11,
+              "the staged planes are two runs of consecutive planes");
+// A particle's inputs in that order, from a lane's column of the stage or
+// straight from the pool.
+struct StagedIn {
+  const float* col;
+  __device__ __forceinline__ float f(int q) const { return col[32 * q]; }
+  __device__ __forceinline__ uint32_t mat() const { return __float_as_uint(f(kStagedInputs - 1)) & 7u; }
+};
+struct PoolIn {
+  const PoolDev& p;
+  uint32_t s;
+  __device__ __forceinline__ float f(int q) const { return plane(p, q < 3 ? PX + q : F0 + q - 3)[s]; }
+  __device__ __forceinline__ uint32_t mat() const { return p.meta[s] & 7u; }
+};
+constexpr int kInMass = 12, kInVol = 13, kInJp = 14;
 // Lattice x of a record that deposits nothing: outside every grid.
 constexpr float kOffGrid = 1.0e30f;
 static_assert(PY == PX + 1 && PZ == PX + 2 && MASS == F0 + 9 && VOL == F0 + 10 && JP == F0 + 11,
               "the staged planes are two runs of consecutive planes");
 
-// The CTA-uniform values of the item a gather CTA is on, kept in shared
-// memory so that they hold no registers through the particle computation:
-// the scene's status word, the 8^3 velocity block origin, whether this
-// substep publishes v and C, and the item's slot range.
+// The uniform values of the unit a gather warp is on, kept in shared memory so
+// that they hold no registers through the particle computation: the scene's
+// status word, the 8^3 velocity block origin, whether this substep publishes v
+// and C, and the unit's slot range.
 struct GatherCtx {
   uint32_t* status;
   int rx, ry, rz;
@@ -184,56 +205,27 @@ struct GatherCtx {
   uint32_t start, count;
 };
 
-// One particle of an item: G2P + F update + return mapping (MODE != kRecord)
-// and the scatter record (MODE != kG2P), returned in rec.  ctx holds the
-// item's uniform values; vblock is the staged 8^3-node velocity block of the
-// item's tile (origin node ctx.rx, ctx.ry, ctx.rz); fallback is a 12-float
-// shared-memory slot of this thread for gather_global.  `in` (kStagedInputs
-// words kGatherThreads apart, or null) holds the particle's inputs in the
-// staged order above, copied to shared memory ahead of time (k_g2p); null
-// reads them from the pool.
-template <int MODE, bool WRITE_KEYS, class SR>
+// One particle: G2P + F update + return mapping (MODE != kRecord) and the
+// scatter record (MODE != kG2P), returned in rec.  ctx holds the unit's
+// uniform values; vblock is the staged 8^3-node velocity block of its tile
+// (origin node ctx.rx, ctx.ry, ctx.rz).  Inputs are read when they are needed
+// (mass, volume, J_p and material would hold four registers through the G2P
+// and the SVD); `done` is called after the last of them.
+template <int MODE, bool WRITE_KEYS, class SR, class IN, class DONE>
 __device__ __forceinline__ void particle_step(const PoolDev& p, const SceneDev& sc, uint32_t s, const GatherCtx& ctx,
-                                              const float4* __restrict__ vblock, float* fallback, SR stol, int sweeps,
-                                              int reuse_svd, float4 (&rec)[4], const float* __restrict__ in = nullptr) {
+                                              const float4* __restrict__ vblock, SR stol, int sweeps,
+                                              const IN in, DONE&& done, float4 (&rec)[4]) {
   constexpr bool kGather = MODE != kRecord;
   constexpr bool kScatter = MODE != kG2P;
-  float x, y, z, F[9], jp, mass, vol;
-  uint32_t mat;
-  if (in) {
-    x = in[0];
-    y = in[kGatherThreads];
-    z = in[2 * kGatherThreads];
-#pragma unroll
-    for (int i = 0; i < 9; ++i) F[i] = in[(3 + i) * kGatherThreads];
-    mass = in[12 * kGatherThreads];
-    vol = in[13 * kGatherThreads];
-    jp = in[14 * kGatherThreads];
-    mat = __float_as_uint(in[15 * kGatherThreads]) & 7u;
-  } else {
-    x = plane(p, PX)[s];
-    y = plane(p, PY)[s];
-    z = plane(p, PZ)[s];
-#pragma unroll
-    for (int i = 0; i < 9; ++i) F[i] = plane(p, F0 + i)[s];
-    jp = plane(p, JP)[s];
-    mass = plane(p, MASS)[s];
-    vol = plane(p, VOL)[s];
-    mat = p.meta[s] & 7u;
-  }
+  float x, y, z, F[9], jp;
   float v[3], C[9];
   bool ok = true;
   SvdOut<SR> svd;
   if constexpr (kGather) {
     // ---- g2p (mpm.wgsl:1242-1353) ----
-    const float xp[3] = {lattice_pos(x, sc.ox, sc.inv_dx), lattice_pos(y, sc.oy, sc.inv_dx),
-                         lattice_pos(z, sc.oz, sc.inv_dx)};
-    const float chk[16] = {x, y, z, jp, F[0], F[1], F[2], F[3], F[4], F[5], F[6], F[7], F[8], xp[0], xp[1], xp[2]};
-    if (!all_finite(chk)) {
-      atomicOr(ctx.status, kFaultNumerical);
-      ok = false;
-    }
-    if (ok) {
+    const float xp[3] = {lattice_pos(in.f(0), sc.ox, sc.inv_dx), lattice_pos(in.f(1), sc.oy, sc.inv_dx),
+                         lattice_pos(in.f(2), sc.oz, sc.inv_dx)};
+    {
       float w[3][3], d[3][3];
       int base[3];
       const int win[3] = {sc.winx, sc.winy, sc.winz};
@@ -253,48 +245,106 @@ __device__ __forceinline__ void particle_step(const PoolDev& p, const SceneDev& 
       float vs[3] = {0.f, 0.f, 0.f};
       float G[9];
       if (inside) {
-#pragma unroll
-        for (int i = 0; i < 9; ++i) G[i] = 0.f;
         const float4* __restrict__ blk = &vblock[lx0 + 8 * ly0 + 64 * lz0];
+        if constexpr (sizeof(SR) == 4) {
+          // In pairs (one instruction for two sums) in the FP32 form; the FP64
+          // form has no registers left for them (it spilled 164 bytes and the
+          // 16M gather went from 1.19 to 1.36 ms, where the FP32 one gained 6%).
+          // The sums over k, then j, then i of the products with the weights
+          // (and, for one axis at a time, with the offset d), the components in
+          // pairs: (x, y) of sum w gv, z of it beside z of sum w d_z gv, (x, y)
+          // of the latter.
+          float2 v01 = make_float2(0.f, 0.f), v2z2 = v01, z01 = v01, x01 = v01, y01 = v01;
+          float x2 = 0.f, y2 = 0.f;
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          float si[3] = {0.f, 0.f, 0.f}, syi[3] = {0.f, 0.f, 0.f}, szi[3] = {0.f, 0.f, 0.f};
+          for (int i = 0; i < 3; ++i) {
+            float2 s01 = make_float2(0.f, 0.f), s2t2 = s01, t01 = s01, u01 = s01;
+            float u2 = 0.f;
 #pragma unroll
-          for (int j = 0; j < 3; ++j) {
-            float sj[3] = {0.f, 0.f, 0.f}, szj[3] = {0.f, 0.f, 0.f};
+            for (int j = 0; j < 3; ++j) {
+              float2 a01 = make_float2(0.f, 0.f), a2b2 = a01, b01 = a01;
 #pragma unroll
-            for (int kk = 0; kk < 3; ++kk) {
-              const float4 g = blk[i + 8 * j + 64 * kk];
-              const float wk = w[2][kk];
-              sj[0] += wk * g.x;
-              sj[1] += wk * g.y;
-              sj[2] += wk * g.z;
-              const float wdk = wk * d[2][kk];
-              szj[0] += wdk * g.x;
-              szj[1] += wdk * g.y;
-              szj[2] += wdk * g.z;
+              for (int kk = 0; kk < 3; ++kk) {
+                const float4 g = blk[i + 8 * j + 64 * kk];
+                const float wk = w[2][kk], wd = wk * d[2][kk];
+                const float2 gxy = make_float2(g.x, g.y);
+                a01 = fma2(make_float2(wk, wk), gxy, a01);
+                a2b2 = fma2(make_float2(wk, wd), make_float2(g.z, g.z), a2b2);
+                b01 = fma2(make_float2(wd, wd), gxy, b01);
+              }
+              const float wj = w[1][j], wd = wj * d[1][j];
+              const float2 wj2 = make_float2(wj, wj);
+              s01 = fma2(wj2, a01, s01);
+              s2t2 = fma2(wj2, a2b2, s2t2);
+              t01 = fma2(wj2, b01, t01);
+              u01 = fma2(make_float2(wd, wd), a01, u01);
+              u2 = fmaf(wd, a2b2.x, u2);
             }
-            const float wj = w[1][j];
-            const float wdj = wj * d[1][j];
+            const float wi = w[0][i], wd = wi * d[0][i];
+            const float2 wi2 = make_float2(wi, wi);
+            v01 = fma2(wi2, s01, v01);
+            v2z2 = fma2(wi2, s2t2, v2z2);
+            z01 = fma2(wi2, t01, z01);
+            x01 = fma2(make_float2(wd, wd), s01, x01);
+            x2 = fmaf(wd, s2t2.x, x2);
+            y01 = fma2(wi2, u01, y01);
+            y2 = fmaf(wi, u2, y2);
+          }
+          vs[0] = v01.x;
+          vs[1] = v01.y;
+          vs[2] = v2z2.x;
+          G[0] = x01.x;
+          G[1] = x01.y;
+          G[2] = x2;
+          G[3] = y01.x;
+          G[4] = y01.y;
+          G[5] = y2;
+          G[6] = z01.x;
+          G[7] = z01.y;
+          G[8] = v2z2.y;
+        } else {
+#pragma unroll
+          for (int i = 0; i < 9; ++i) G[i] = 0.f;
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            float si[3] = {0.f, 0.f, 0.f}, syi[3] = {0.f, 0.f, 0.f}, szi[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+              float sj[3] = {0.f, 0.f, 0.f}, szj[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+              for (int kk = 0; kk < 3; ++kk) {
+                const float4 g = blk[i + 8 * j + 64 * kk];
+                const float wk = w[2][kk];
+                sj[0] += wk * g.x;
+                sj[1] += wk * g.y;
+                sj[2] += wk * g.z;
+                const float wdk = wk * d[2][kk];
+                szj[0] += wdk * g.x;
+                szj[1] += wdk * g.y;
+                szj[2] += wdk * g.z;
+              }
+              const float wj = w[1][j];
+              const float wdj = wj * d[1][j];
+#pragma unroll
+              for (int r = 0; r < 3; ++r) {
+                si[r] += wj * sj[r];
+                syi[r] += wdj * sj[r];
+                szi[r] += wj * szj[r];
+              }
+            }
+            const float wi = w[0][i];
+            const float wdi = wi * d[0][i];
 #pragma unroll
             for (int r = 0; r < 3; ++r) {
-              si[r] += wj * sj[r];
-              syi[r] += wdj * sj[r];
-              szi[r] += wj * szj[r];
+              vs[r] += wi * si[r];
+              G[r] += wdi * si[r];      // column x
+              G[3 + r] += wi * syi[r];  // column y
+              G[6 + r] += wi * szi[r];  // column z
             }
-          }
-          const float wi = w[0][i];
-          const float wdi = wi * d[0][i];
-#pragma unroll
-          for (int r = 0; r < 3; ++r) {
-            vs[r] += wi * si[r];
-            G[r] += wdi * si[r];      // column x
-            G[3 + r] += wi * syi[r];  // column y
-            G[6 + r] += wi * szi[r];  // column z
           }
         }
       } else {
-        float* slot = fallback;
+        float slot[12];
         gather_global(p.vel, sc, p.tile_slot, xp[0], xp[1], xp[2], slot);
 #pragma unroll
         for (int r = 0; r < 3; ++r) vs[r] = slot[r];
@@ -307,7 +357,7 @@ __device__ __forceinline__ void particle_step(const PoolDev& p, const SceneDev& 
       v[0] = vs[0];
       v[1] = vs[1];
       v[2] = vs[2];
-      const MatDev& md = sc.mat[mat];
+      const MatDev& md = sc.mat[in.mat()];
       if (md.rheo == 2) {
         v[0] *= md.vfac;
         v[1] *= md.vfac;
@@ -315,10 +365,25 @@ __device__ __forceinline__ void particle_step(const PoolDev& p, const SceneDev& 
 #pragma unroll
         for (int i = 0; i < 9; ++i) C[i] *= md.afac;
       }
+      x = in.f(0);
+      y = in.f(1);
+      z = in.f(2);
+#pragma unroll
+      for (int i = 0; i < 9; ++i) F[i] = in.f(3 + i);
       float np[3] = {x + sc.dt * v[0], y + sc.dt * v[1], z + sc.dt * v[2]};
-      const float chk2[15] = {np[0], v[0], np[1], v[1], np[2], v[2], C[0], C[1], C[2],
-                              C[3],  C[4], C[5],  C[6], C[7],  C[8]};
-      if (!all_finite(chk2)) {
+      // F <- (I + dt C) F
+      float A[9];
+#pragma unroll
+      for (int i = 0; i < 9; ++i) A[i] = sc.dt * C[i] + ((i % 4 == 0) ? 1.f : 0.f);
+      float Fn[9];
+      matmul(A, F, Fn);
+      jp = in.f(kInJp);
+      // One test for the reference's three (the inputs, the new x, v and C,
+      // the new F; each of which leaves the particle as it was): a non-finite
+      // position or velocity reaches np, a non-finite F or C reaches Fn.
+      const float chk[16] = {np[0], np[1], np[2], jp,    xp[0], xp[1], xp[2], Fn[0],
+                             Fn[1], Fn[2], Fn[3], Fn[4], Fn[5], Fn[6], Fn[7], Fn[8]};
+      if (!all_finite(chk)) {
         atomicOr(ctx.status, kFaultNumerical);
         ok = false;
       }
@@ -328,16 +393,7 @@ __device__ __forceinline__ void particle_step(const PoolDev& p, const SceneDev& 
           if (np[a] < sc.lo[a] || np[a] > sc.hi[a]) v[a] = 0.f;
           np[a] = clampf(np[a], sc.lo[a], sc.hi[a]);
         }
-        // F <- (I + dt C) F
-        float A[9];
-#pragma unroll
-        for (int i = 0; i < 9; ++i) A[i] = sc.dt * C[i] + ((i % 4 == 0) ? 1.f : 0.f);
-        float Fn[9];
-        matmul(A, F, Fn);
-        if (!all_finite(Fn)) {
-          atomicOr(ctx.status, kFaultNumerical);
-          ok = false;
-        } else {
+        {
           x = np[0];
           y = np[1];
           z = np[2];
@@ -352,37 +408,24 @@ __device__ __forceinline__ void particle_step(const PoolDev& p, const SceneDev& 
           bool changed = true;
           const SR s_trial[3] = {svd.s[0], svd.s[1], svd.s[2]};
           if (plasticity_project<SR>(svd, md, jp_new, changed)) {
-            // FP32 mode rebuilds F = U s V^T every substep (the
-            // reference).  The FP64-SVD mode keeps the trial F when the
-            // return mapping left every singular value unchanged, and
-            // otherwise adds U diag(s - s_trial) V^T to it: the same F as
-            // U s V^T in exact arithmetic (F = U s_trial V^T), with the
-            // FP32 rounding of U and V scaled by the (small) change in s
-            // instead of by F.
-            float Fr[9];
-            const bool rebuild = sizeof(SR) == 4 || changed;
-            if (rebuild) {
+            // The trial F stays when the return mapping left every singular
+            // value unchanged; otherwise U diag(s - s_trial) V^T is added to
+            // it: the reference's F = U s V^T in exact arithmetic (F = U
+            // s_trial V^T), with the FP32 rounding of U and V scaled by the
+            // (small) change in s instead of by F.  Finite: s lies in [0.05,
+            // 20] and F = U s_trial V^T.
+            if (changed) {
               float ds[3];
 #pragma unroll
-              for (int i = 0; i < 3; ++i) ds[i] = sizeof(SR) == 4 ? (float)svd.s[i] : (float)(svd.s[i] - s_trial[i]);
+              for (int i = 0; i < 3; ++i) ds[i] = (float)(svd.s[i] - s_trial[i]);
 #pragma unroll
               for (int c = 0; c < 3; ++c)
 #pragma unroll
                 for (int r = 0; r < 3; ++r)
-                  Fr[3 * c + r] = (sizeof(SR) == 4 ? 0.0f : F[3 * c + r]) + (svd.u[r] * ds[0]) * svd.v[c] +
-                                  (svd.u[3 + r] * ds[1]) * svd.v[3 + c] + (svd.u[6 + r] * ds[2]) * svd.v[6 + c];
+                  F[3 * c + r] += (svd.u[r] * ds[0]) * svd.v[c] + (svd.u[3 + r] * ds[1]) * svd.v[3 + c] +
+                                  (svd.u[6 + r] * ds[2]) * svd.v[6 + c];
             }
-            // the FP32 copy must be finite too (an FP64 value beyond FP32 range)
-            if (!rebuild || all_finite(Fr)) {
-              if (rebuild) {
-#pragma unroll
-                for (int i = 0; i < 9; ++i) F[i] = (float)Fr[i];
-              }
-              jp = jp_new;
-            } else {
-              atomicOr(ctx.status, kFaultNumerical);
-              ok = false;
-            }
+            jp = jp_new;
           } else {
             atomicOr(ctx.status, kFaultNumerical);
             ok = false;
@@ -416,11 +459,17 @@ __device__ __forceinline__ void particle_step(const PoolDev& p, const SceneDev& 
     // reference's g2p checks, mpm.wgsl:1247-1255, moved to the first
     // launch of the call so that a non-finite upload latches before
     // anything moves).
+    x = in.f(0);
+    y = in.f(1);
+    z = in.f(2);
+#pragma unroll
+    for (int i = 0; i < 9; ++i) F[i] = in.f(3 + i);
     v[0] = plane(p, VX)[s];
     v[1] = plane(p, VY)[s];
     v[2] = plane(p, VZ)[s];
 #pragma unroll
     for (int i = 0; i < 9; ++i) C[i] = plane(p, C0 + i)[s];
+    jp = in.f(kInJp);
     bool fin = finitef(x) && finitef(y) && finitef(z) && finitef(jp) && finitef(v[0]) && finitef(v[1]) &&
                finitef(v[2]) && finitef(lattice_pos(x, sc.ox, sc.inv_dx)) &&
                finitef(lattice_pos(y, sc.oy, sc.inv_dx)) && finitef(lattice_pos(z, sc.oz, sc.inv_dx));
@@ -431,6 +480,9 @@ __device__ __forceinline__ void particle_step(const PoolDev& p, const SceneDev& 
       ok = false;
     }
   }
+  const uint32_t mat = in.mat();
+  const float mass = in.f(kInMass), vol = in.f(kInVol);
+  done();
   if constexpr (kScatter || WRITE_KEYS) {
     // lattice coordinates of the new position
     const float xq[3] = {lattice_pos(x, sc.ox, sc.inv_dx), lattice_pos(y, sc.oy, sc.inv_dx),
@@ -447,7 +499,7 @@ __device__ __forceinline__ void particle_step(const PoolDev& p, const SceneDev& 
 #pragma unroll
       for (int i = 0; i < 9; ++i) Bd[i] = 0.f;
       if (ok) {
-        if (!kGather || !reuse_svd) {
+        if constexpr (!kGather) {
           SR Fs[9];
 #pragma unroll
           for (int i = 0; i < 9; ++i) Fs[i] = (SR)F[i];
@@ -481,101 +533,138 @@ __device__ __forceinline__ void particle_step(const PoolDev& p, const SceneDev& 
   }
 }
 
-// MODE: kRecord (no gather: validate the state and compute B from the SVD of
-// F — the first substep of a call), kG2P (gather + return mapping, the last
-// substep of a call), kG2PRecord (gather + return mapping + B for the next
-// scatter, with the return mapping's SVD reused).
+// A gather warp's shared memory: the velocity block, the particle inputs of
+// its lanes' next round ([input][lane], the staged order), the scene record.
+template <bool GATHER>
+struct __align__(128) GatherWarp {
+  float4 vel[GATHER ? kRegionNodes : 1];
+  float in[kStagedInputs][32];
+  SceneDev sc;
+  GatherCtx ctx;
+  uint32_t scene;   // scene whose record sc holds
+  uint32_t parity;  // of the velocity block's next arrival
+  uint64_t bar;
+};
+
+// MODE: kRecord (no gather: validate the state and compute the record from the
+// SVD of F — the first substep of a call), kG2P (gather + return mapping, the
+// last substep of a call), kG2PRecord (gather + return mapping + the record
+// for the next scatter, with the return mapping's SVD reused).
+//
+// Every warp works alone: it takes units (a piece of a tile's particles) from
+// the list, its first by its index and each later one from the counter, with
+// the velocity block of the unit's tile fetched into its own shared memory by
+// one TMA box, and shares no barrier with the other warps of its CTA.
+// What bounds it: instruction issue (60% of the slots; 64 warp instructions a
+// particle of mixed materials) and, behind that, instruction fetch -- the
+// kernel was 55 KB, of which a second SVD for a case that never came was 13 --
+// and the dependent chains of the SVD; a quarter of the DRAM rate.  Against a
+// CTA per tile with a barrier per item: 1.26 -> 1.19 ms at 16M particles (FP64
+// SVD, 256^3), 333 -> 278 us at 4M and 63 -> 52 us at 500k (FP32).
 template <int MODE, bool WRITE_KEYS, class SR>
-__global__ void __launch_bounds__(kGatherThreads, 5) k_g2p(PoolDev p, double tol, int sweeps, int reuse_svd,
+__global__ void __launch_bounds__(kGatherThreads, 5) k_g2p(PoolDev p, double tol, int sweeps,
                                                             int publish_all) {
   constexpr bool kGather = MODE != kRecord;
   constexpr bool kScatter = MODE != kG2P;
-  __shared__ __align__(16) SceneDev s_sc;
-  __shared__ __align__(16) SharedGather s_gath;
-  __shared__ uint32_t s_fault;
-  __shared__ GatherCtx s_ctx;
-  __shared__ uint32_t s_it_next;
-  // Particle inputs of this round and the next (cp.async double buffer):
-  // [buffer][input][thread], the inputs in the staged order.
-  __shared__ __align__(16) float s_in[2][kStagedInputs][kGatherThreads];
-  // this SVD form's range of the work list: FP32-SVD items, then FP64-SVD items
-  const uint32_t n32 = p.n_items[0];
-  const uint32_t it_lo = sizeof(SR) == 8 ? n32 : 0u;
-  const uint32_t it_hi = sizeof(SR) == 8 ? n32 + p.n_items[1] : n32;
+  constexpr uint32_t kWarps = kGatherThreads / 32;
+  __shared__ GatherWarp<kGather> s_warp[kWarps];
+  const uint32_t lane = threadIdx.x & 31u;
+  GatherWarp<kGather>& w = s_warp[threadIdx.x >> 5];
+  if (lane == 0) {
+    w.scene = 0xffffffffu;
+    w.parity = 0;
+    mbar_init(&w.bar, 1);
+    fence_mbar_init();
+  }
+  __syncwarp();
+  launch_next();
+  wait_previous();
+  // this SVD form's range of the list: units of FP32-SVD scenes, then FP64-SVD
+  const uint32_t n32 = p.n_units[0];
+  const uint32_t lo = sizeof(SR) == 8 ? n32 : 0u;
+  const uint32_t hi = sizeof(SR) == 8 ? n32 + p.n_units[1] : n32;
   const SR stol = (SR)tol;
-  uint32_t s_sc_scene = 0xffffffffu;  // scene whose record s_sc holds
-  for (uint32_t it = it_lo + blockIdx.x; it < it_hi;) {
-    const Item item = p.items[item_slot(p, n32, it)];
-    // this CTA's next item, taken now and read by all after the item's work
-    if (threadIdx.x == 0) s_it_next = it_lo + gridDim.x + atomicAdd(p.work, 1u);
-    // A thread's particles come kGatherThreads apart; the inputs of its
-    // next particle are copied to shared memory (cp.async) while it computes
-    // this one, and those of its first are requested here, so that their
-    // loads overlap the velocity block's.
-    const uint32_t tid = threadIdx.x;
-    auto fetch = [&](uint32_t k, int b, uint32_t start, uint32_t count) {
+  // first units spread over the CTAs, so that a short list uses every SM
+  for (uint32_t u = lo + (threadIdx.x >> 5) * gridDim.x + blockIdx.x; u < hi;) {
+    const Item unit = p.units[unit_slot(p, n32, u)];
+    uint32_t next = 0;  // this warp's next unit, taken now and read after this one's work
+    if (lane == 0) next = lo + kWarps * gridDim.x + atomicAdd(p.work + (sizeof(SR) == 8 ? kWorkGather64 : kWorkGather32), 1u);
+    // The inputs of a lane's next particle are copied to shared memory
+    // (cp.async) from the moment this one's are consumed; those of its first
+    // are requested here, so that their loads overlap the velocity block's.
+    auto fetch = [&](uint32_t k, uint32_t start, uint32_t count) {
       if (k < count) {
         const uint32_t s = start + k;
         // walk the planes with one pointer: PX..PZ, then F0..JP
         const size_t cap = p.cap;
         const float* src = p.planes + s;
 #pragma unroll
-        for (int q = 0; q < 3; ++q, src += cap) cp_async4(&s_in[b][q][tid], src);
+        for (int q = 0; q < 3; ++q, src += cap) cp_async4(&w.in[q][lane], src);
         src += (size_t)(F0 - 3) * cap;
 #pragma unroll
-        for (int q = 3; q < kStagedInputs - 1; ++q, src += cap) cp_async4(&s_in[b][q][tid], src);
-        cp_async4(&s_in[b][kStagedInputs - 1][tid], p.meta + s);
+        for (int q = 3; q < kStagedInputs - 1; ++q, src += cap) cp_async4(&w.in[q][lane], src);
+        cp_async4(&w.in[kStagedInputs - 1][lane], p.meta + s);
       }
-      cp_async_commit();
     };
-    fetch(tid, 0, item.start, item.count);
-    // The scene record goes to shared memory when the item's scene differs
-    // from the last item's (consecutive items of a CTA mostly share one):
-    // the velocity staging below reads the geometry from there, so a new
-    // record is published by a barrier first.
-    if (item.scene != s_sc_scene) {
-      const uint32_t* src = reinterpret_cast<const uint32_t*>(p.scenes + item.scene);
-      uint32_t* dst = reinterpret_cast<uint32_t*>(&s_sc);
-      for (int k = threadIdx.x; k < (int)(sizeof(SceneDev) / 4); k += kGatherThreads) dst[k] = src[k];
-      s_sc_scene = item.scene;
-      __syncthreads();
-    }
-    const SceneDev& sc = s_sc;
-    const uint32_t w = sc.w;
-    const uint32_t tx = item.tile % w, ty = (item.tile / w) % w, tz = item.tile / (w * w);
-    const int rx = 4 * (int)tx - 1, ry = 4 * (int)ty - 1, rz = 4 * (int)tz - 1;
-    if (threadIdx.x == 0) {
-      uint32_t* status = p.status + (size_t)sc.status * kStatusWords;
-      // a latched fault, a spent substep budget or a retired scene: stand still
-      s_fault = (scene_frozen(status) || !sc.live) ? 1u : 0u;
-      s_ctx = GatherCtx{status, rx, ry, rz, (publish_all || budget_ends(status)) ? 1u : 0u, item.start, item.count};
-    }
-    if constexpr (kGather) {
-      // Stage the 8^3-node velocity block (out-of-grid nodes read as zero),
-      // the four loads of a thread in flight together.
-      constexpr int kPer = kRegionNodes / kGatherThreads;
-      static_assert(kPer * kGatherThreads == kRegionNodes, "the block splits evenly over the CTA");
-      float4 g[kPer];
-#pragma unroll
-      for (int q = 0; q < kPer; ++q) {
-        const int r = (int)threadIdx.x + q * kGatherThreads;
-        const int64_t c = node_index(sc, p.tile_slot, rx + (r & 7), ry + ((r >> 3) & 7), rz + (r >> 6));
-        g[q] = c >= 0 ? __ldg(&p.vel[c]) : make_float4(0.f, 0.f, 0.f, 0.f);
+    fetch(lane, unit.start, unit.count);
+    if (unit.scene != w.scene) {
+      const uint32_t* src = reinterpret_cast<const uint32_t*>(p.scenes + unit.scene);
+      uint32_t* dst = reinterpret_cast<uint32_t*>(&w.sc);
+      for (uint32_t k = lane; k < sizeof(SceneDev) / 4; k += 32) dst[k] = src[k];
+      __syncwarp();
+      if (lane == 0) {
+        w.scene = unit.scene;
+        // the scene's tensor map was written by a copy before this launch
+        if (kGather) fence_tensormap(p.vel_maps + unit.scene);
       }
-#pragma unroll
-      for (int q = 0; q < kPer; ++q) s_gath.vel[(int)threadIdx.x + q * kGatherThreads] = g[q];
+      __syncwarp();
     }
-    __syncthreads();
-    const bool faulted = s_fault != 0;
-    if (!faulted) {
-      int b = 0;
-      for (uint32_t k = tid; k < s_ctx.count; k += kGatherThreads, b ^= 1) {
-        fetch(k + kGatherThreads, b ^ 1, s_ctx.start, s_ctx.count);
-        cp_async_wait<1>();
-        const uint32_t s = s_ctx.start + k;
+    const SceneDev& sc = w.sc;
+    uint32_t* status = p.status + (size_t)sc.status * kStatusWords;
+    // a latched fault, a spent substep budget or a retired scene: stand still
+    if (!scene_frozen(status) && sc.live) {
+      const uint32_t tw = sc.w;
+      const uint32_t tx = unit.tile % tw, ty = (unit.tile / tw) % tw, tz = unit.tile / (tw * tw);
+      const int rx = 4 * (int)tx - 1, ry = 4 * (int)ty - 1, rz = 4 * (int)tz - 1;
+      if (lane == 0)
+        w.ctx = GatherCtx{status, rx, ry, rz, (publish_all || budget_ends(status)) ? 1u : 0u, unit.start, unit.count};
+      if constexpr (kGather) {
+        // Stage the 8^3-node velocity block (out-of-grid nodes read as zero).
+        if (sc.tile_cap == 0 && sc.n >= (uint32_t)kRegion) {
+          if (lane == 0) {
+            fence_proxy_async_smem();  // the lanes' reads of the block are done (__syncwarp below)
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(&w.bar)),
+                         "r"((uint32_t)sizeof(w.vel))
+                         : "memory");
+            tma_load_box(w.vel, p.vel_maps + unit.scene, 4 * rx, ry, rz, &w.bar);
+          }
+          const uint32_t parity = w.parity;
+          if (!mbar_wait_bounded(&w.bar, parity)) {
+            // The copy did not arrive: report it, wait once more (bounded)
+            // for it and stop this warp.
+            if (lane == 0) atomicOr(status, kFaultDeviceWait);
+            mbar_wait_bounded(&w.bar, parity);
+            cp_async_wait_all();
+            return;
+          }
+          __syncwarp();
+          if (lane == 0) w.parity = parity ^ 1u;
+        } else {
+          for (uint32_t r = lane; r < (uint32_t)kRegionNodes; r += 32) {
+            const int64_t c =
+                node_index(sc, p.tile_slot, rx + (int)(r & 7u), ry + (int)((r >> 3) & 7u), rz + (int)(r >> 6));
+            w.vel[r] = c >= 0 ? __ldg(&p.vel[c]) : make_float4(0.f, 0.f, 0.f, 0.f);
+          }
+        }
+      }
+      __syncwarp();
+      for (uint32_t k = lane; k < w.ctx.count; k += 32) {
+        cp_async_wait_all();
+        const uint32_t s = w.ctx.start + k;
         float4 rec[4];
-        particle_step<MODE, WRITE_KEYS, SR>(p, sc, s, s_ctx, s_gath.vel, s_gath.fallback[threadIdx.x], stol, sweeps,
-                                            reuse_svd, rec, &s_in[b][0][tid]);
+        particle_step<MODE, WRITE_KEYS, SR>(
+            p, sc, s, w.ctx, w.vel, stol, sweeps, StagedIn{&w.in[0][lane]},
+            [&] { fetch(k + 32u, w.ctx.start, w.ctx.count); }, rec);
         if constexpr (kScatter) {
           float4* r4 = reinterpret_cast<float4*>(p.rec) + 4 * (size_t)s;
           r4[0] = rec[0];
@@ -585,12 +674,9 @@ __global__ void __launch_bounds__(kGatherThreads, 5) k_g2p(PoolDev p, double tol
         }
       }
     }
-    cp_async_wait<0>();
-    // s_it_next was published by the barrier after the staging; thread 0
-    // overwrites it only after the barrier below
-    const uint32_t next = s_it_next;
-    __syncthreads();
-    it = next;
+    cp_async_wait_all();
+    __syncwarp();
+    u = __shfl_sync(0xffffffffu, next, 0);
   }
 }
 
@@ -646,6 +732,7 @@ __device__ __noinline__ void deposit_global(float4 c0, float4 c1, float4 c2, flo
     base[a] = (int)bf - win[a];
     quad_weights(xp[a] - bf, wgt[a]);
   }
+#pragma unroll 1
   for (int q = 0; q < 27; ++q) {
     const int i = q / 9, j = (q / 3) % 3, k = q % 3;
     const int64_t c = node_index(sc, tile_slot, base[0] + i, base[1] + j, base[2] + k);
@@ -900,10 +987,12 @@ __global__ void __launch_bounds__(kScatterThreads, 4) k_p2g(PoolDev p, const __g
   __shared__ __align__(16) Item s_desc;     // descriptor of the next item, copied ahead
   __shared__ ScatterItem s_item[2];         // this item's frame and the next one's
   __shared__ uint32_t s_next;
+  launch_next();
+  clear_scatter_shared(ss, kScatterThreads);
+  wait_previous();
   const uint32_t n32 = p.n_items[0];
   const uint32_t n_items = n32 + p.n_items[1];
   if (blockIdx.x >= n_items) return;
-  clear_scatter_shared(ss, kScatterThreads);
   // Thread 0 stages an item (of 1..kStageMax particles) as ceil(count / 64)
   // tiles; rows past the item are loaded but not read.
   auto stage = [&](const Item& nx) {
@@ -934,7 +1023,7 @@ __global__ void __launch_bounds__(kScatterThreads, 4) k_p2g(PoolDev p, const __g
     // the deposit and stages its records after it, so that no thread waits
     // for the counter or the descriptor.
     uint32_t next = 0;
-    if (threadIdx.x == 0) next = gridDim.x + atomicAdd(p.work + 1, 1u);
+    if (threadIdx.x == 0) next = gridDim.x + atomicAdd(p.work + kWorkScatter, 1u);
     const uint32_t share = core_share(p.item_order + (size_t)f.slot * 64);
     const bool staged = f.count - 1u < (uint32_t)kStageMax;
     const bool ok = staged && mbar_wait_bounded(&s_bar, parity);
@@ -983,7 +1072,7 @@ __global__ void __launch_bounds__(kScatterThreads, 4) k_p2g(PoolDev p, const __g
 // deposit); a particle that faults during the gather deposits nothing (m = 0
 // in its record).  The scene is frozen from the next substep on.
 template <bool WRITE_KEYS, class SR>
-__global__ void __launch_bounds__(kFusedThreads, 2) k_g2p2g(PoolDev p, double tol, int sweeps, int reuse_svd,
+__global__ void __launch_bounds__(kFusedThreads, 2) k_g2p2g(PoolDev p, double tol, int sweeps,
                                                               int acc_out) {
   extern __shared__ __align__(16) float4 s_stage[];  // kStageMax records, 64-byte swizzle
   __shared__ __align__(16) SceneDev s_sc;
@@ -991,13 +1080,15 @@ __global__ void __launch_bounds__(kFusedThreads, 2) k_g2p2g(PoolDev p, double to
   __shared__ ScatterShared ss;
   __shared__ ScatterItem s_item;
   __shared__ GatherCtx s_ctx;
+  const SR stol = (SR)tol;
+  launch_next();
+  clear_scatter_shared(ss, kFusedThreads);
+  if (threadIdx.x == 0) s_item.sc = nullptr;
+  wait_previous();
   // this SVD form's range of the work list: FP32-SVD items, then FP64-SVD items
   const uint32_t n32 = p.n_items[0];
   const uint32_t it_lo = sizeof(SR) == 8 ? n32 : 0u;
   const uint32_t it_hi = sizeof(SR) == 8 ? n32 + p.n_items[1] : n32;
-  const SR stol = (SR)tol;
-  clear_scatter_shared(ss, kFusedThreads);
-  if (threadIdx.x == 0) s_item.sc = nullptr;
   for (uint32_t it = it_lo + blockIdx.x; it < it_hi; it += gridDim.x) {
     const uint32_t slot = item_slot(p, n32, it);
     const Item item = p.items[slot];
@@ -1029,11 +1120,10 @@ __global__ void __launch_bounds__(kFusedThreads, 2) k_g2p2g(PoolDev p, double to
     const bool live = s_item.live != 0u;
     if (live) {
       for (uint32_t k = threadIdx.x; k < item.count; k += kFusedThreads) {
+        const uint32_t s = item.start + k;
         float4 rec[4];
-        // the record's own stage slot is the scratch of gather_global
-        particle_step<kG2PRecord, WRITE_KEYS, SR>(p, s_sc, item.start + k, s_ctx, s_vel,
-                                                  reinterpret_cast<float*>(s_stage + 4 * (size_t)k), stol, sweeps,
-                                                  reuse_svd, rec);
+        particle_step<kG2PRecord, WRITE_KEYS, SR>(p, s_sc, s, s_ctx, s_vel, stol, sweeps, PoolIn{p, s}, [] {},
+                                                  rec);
         stage_store(s_stage, k, rec);
       }
       // a thread bins the records it wrote
@@ -1240,24 +1330,26 @@ __global__ void k_combine_det(PoolDev p, const float4* __restrict__ blocks, cons
 // ---------------------------------------------------------------------------
 
 template <int MODE, bool KEYS, class SR>
-static cudaError_t launch_gather_t(const PoolDev& p, double tol, int sweeps, int reuse, int grid, cudaStream_t st,
+static cudaError_t launch_gather_t(const PoolDev& p, double tol, int sweeps, int grid, cudaStream_t st,
                                    bool publish_all) {
-  const cudaError_t e = cudaMemsetAsync(p.work, 0, sizeof(uint32_t), st);
-  if (e != cudaSuccess) return e;
-  k_g2p<MODE, KEYS, SR><<<grid, kGatherThreads, 0, st>>>(p, tol, sweeps, reuse, publish_all ? 1 : 0);
-  return cudaGetLastError();
+  if (MODE == kRecord) {
+    // opens a call, with no grid update before it
+    const cudaError_t e = cudaMemsetAsync(p.work, 0, kWorkWords * sizeof(uint32_t), st);
+    if (e != cudaSuccess) return e;
+  }
+  return launch_dependent(k_g2p<MODE, KEYS, SR>, grid, kGatherThreads, 0, st, p, tol, sweeps, publish_all ? 1 : 0);
 }
 
 cudaError_t launch_gather(int mode, bool write_keys, bool svd_fp64, const PoolDev& p, double tol, int sweeps,
-                          int reuse, int grid, cudaStream_t st, bool publish_all) {
+                          int grid, cudaStream_t st, bool publish_all) {
 #define MPM_DISPATCH(M)                                                                          \
   if (mode == M) {                                                                               \
     if (svd_fp64) {                                                                              \
-      return write_keys ? launch_gather_t<M, true, double>(p, tol, sweeps, reuse, grid, st, publish_all) \
-                        : launch_gather_t<M, false, double>(p, tol, sweeps, reuse, grid, st, publish_all); \
+      return write_keys ? launch_gather_t<M, true, double>(p, tol, sweeps, grid, st, publish_all) \
+                        : launch_gather_t<M, false, double>(p, tol, sweeps, grid, st, publish_all); \
     }                                                                                            \
-    return write_keys ? launch_gather_t<M, true, float>(p, tol, sweeps, reuse, grid, st, publish_all) \
-                      : launch_gather_t<M, false, float>(p, tol, sweeps, reuse, grid, st, publish_all); \
+    return write_keys ? launch_gather_t<M, true, float>(p, tol, sweeps, grid, st, publish_all) \
+                      : launch_gather_t<M, false, float>(p, tol, sweeps, grid, st, publish_all); \
   }
   MPM_DISPATCH(kRecord)
   MPM_DISPATCH(kG2P)
@@ -1269,30 +1361,31 @@ cudaError_t launch_gather(int mode, bool write_keys, bool svd_fp64, const PoolDe
 constexpr size_t kFusedStageBytes = (size_t)kStageMax * 64;
 
 template <bool KEYS, class SR>
-static cudaError_t launch_fused_t(const PoolDev& p, double tol, int sweeps, int reuse, int acc_out, int grid,
+static cudaError_t launch_fused_t(const PoolDev& p, double tol, int sweeps, int acc_out, int grid,
                                   cudaStream_t st) {
-  k_g2p2g<KEYS, SR><<<grid, kFusedThreads, kFusedStageBytes, st>>>(p, tol, sweeps, reuse, acc_out);
-  return cudaGetLastError();
+  return launch_dependent(k_g2p2g<KEYS, SR>, grid, kFusedThreads, kFusedStageBytes, st, p, tol, sweeps, acc_out);
 }
 
-cudaError_t launch_fused(bool write_keys, bool svd_fp64, const PoolDev& p, double tol, int sweeps, int reuse,
+cudaError_t launch_fused(bool write_keys, bool svd_fp64, const PoolDev& p, double tol, int sweeps,
                          int acc_out, int grid, cudaStream_t st) {
   if (svd_fp64)
-    return write_keys ? launch_fused_t<true, double>(p, tol, sweeps, reuse, acc_out, grid, st)
-                      : launch_fused_t<false, double>(p, tol, sweeps, reuse, acc_out, grid, st);
-  return write_keys ? launch_fused_t<true, float>(p, tol, sweeps, reuse, acc_out, grid, st)
-                    : launch_fused_t<false, float>(p, tol, sweeps, reuse, acc_out, grid, st);
+    return write_keys ? launch_fused_t<true, double>(p, tol, sweeps, acc_out, grid, st)
+                      : launch_fused_t<false, double>(p, tol, sweeps, acc_out, grid, st);
+  return write_keys ? launch_fused_t<true, float>(p, tol, sweeps, acc_out, grid, st)
+                    : launch_fused_t<false, float>(p, tol, sweeps, acc_out, grid, st);
 }
 
 // stage tiles plus 1 KiB for the alignment of the swizzled stage
 constexpr size_t kStageBytes = (size_t)kStageMax * 64 + 1024;
 static_assert(kStageMax % kStageBoxRows == 0, "the stage holds whole TMA tiles");
 
-bool make_record_map(CUtensorMap* out, const float* rec, uint32_t cap, std::string* err) {
-  using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-  static EncodeFn encode = nullptr;
+using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+static bool encode_map(CUtensorMap* out, int rank, const float* base, const cuuint64_t* dims, const cuuint64_t* strides,
+                       const cuuint32_t* box, CUtensorMapSwizzle swizzle, std::string* err) {
+  static EncodeTiledFn encode = nullptr;
   if (!encode) {
     void* fn = nullptr;
     cudaDriverEntryPointQueryResult q;
@@ -1301,21 +1394,33 @@ bool make_record_map(CUtensorMap* out, const float* rec, uint32_t cap, std::stri
       if (err) *err = "cuTensorMapEncodeTiled is not available from the driver";
       return false;
     }
-    encode = reinterpret_cast<EncodeFn>(fn);
+    encode = reinterpret_cast<EncodeTiledFn>(fn);
   }
-  // records: rows of 16 floats (64 bytes), cap rows; tiles of 64 rows
-  const cuuint64_t dims[2] = {16, cap ? cap : 1};
-  const cuuint64_t strides[1] = {64};
-  const cuuint32_t box[2] = {16, (cuuint32_t)kStageBoxRows};
-  const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = encode(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(rec), dims, strides, box, estr,
-                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  const cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = encode(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, (cuuint32_t)rank, const_cast<float*>(base), dims,
+                            strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     if (err) *err = "cuTensorMapEncodeTiled failed with code " + std::to_string((int)r);
     return false;
   }
   return true;
+}
+
+bool make_record_map(CUtensorMap* out, const float* rec, uint32_t cap, std::string* err) {
+  // records: rows of 16 floats (64 bytes), cap rows; tiles of 64 rows
+  const cuuint64_t dims[2] = {16, cap ? cap : 1};
+  const cuuint64_t strides[1] = {64};
+  const cuuint32_t box[2] = {16, (cuuint32_t)kStageBoxRows};
+  return encode_map(out, 2, rec, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_64B, err);
+}
+
+bool make_velocity_map(CUtensorMap* out, const float4* vel, uint32_t n, std::string* err) {
+  // n^3 nodes of four floats, x fastest; boxes of 8^3 nodes
+  const cuuint64_t dims[3] = {4ull * n, n, n};
+  const cuuint64_t strides[2] = {16ull * n, 16ull * n * n};
+  const cuuint32_t box[3] = {4 * kRegion, kRegion, kRegion};
+  return encode_map(out, 3, reinterpret_cast<const float*>(vel), dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE, err);
 }
 
 // Self-test of the scatter's bounded stage wait: one warp waits, through the
@@ -1346,10 +1451,7 @@ cudaError_t launch_selftest_wait(uint32_t* status, unsigned long long* waited_ns
 }
 
 cudaError_t launch_scatter(const PoolDev& p, const CUtensorMap& rec_map, int acc_out, int grid, cudaStream_t st) {
-  const cudaError_t e = cudaMemsetAsync(p.work + 1, 0, sizeof(uint32_t), st);
-  if (e != cudaSuccess) return e;
-  k_p2g<<<grid, kScatterThreads, kStageBytes, st>>>(p, rec_map, acc_out);
-  return cudaGetLastError();
+  return launch_dependent(k_p2g, grid, kScatterThreads, kStageBytes, st, p, rec_map, acc_out);
 }
 
 cudaError_t launch_scatter_det(const PoolDev& p, float4* blocks, int acc_out, int grid, cudaStream_t st) {

@@ -258,8 +258,9 @@ Group::Group(Engine* e, uint32_t max_scenes_, uint64_t particle_cap, uint64_t ce
   touched[1].alloc(cell_cap / kCellBlock);
   scenes_d.alloc(max_scenes);
   status_d.alloc((size_t)kStatusWords * max_scenes);
-  work_d.alloc(2);
-  n_items.alloc(2);
+  work_d.alloc(kWorkWords);
+  n_items.alloc(4);
+  vel_maps.alloc(max_scenes);
   totals_d.alloc(8);
   MPM_CK(cudaMallocHost((void**)&scenes_h, sizeof(SceneDev) * max_scenes));
   std::memset(scenes_h, 0, sizeof(SceneDev) * max_scenes);
@@ -274,6 +275,7 @@ Group::Group(Engine* e, uint32_t max_scenes_, uint64_t particle_cap, uint64_t ce
   MPM_CK(cudaMemsetAsync(block_scene.ptr, 0xff, block_scene.bytes(), stream));
   MPM_CK(cudaMemsetAsync(status_d.ptr, 0, status_d.bytes(), stream));
   MPM_CK(cudaMemsetAsync(n_items.ptr, 0, n_items.bytes(), stream));
+  MPM_CK(cudaMemsetAsync(work_d.ptr, 0, work_d.bytes(), stream));
   MPM_CK(cudaMemsetAsync(scenes_d.ptr, 0, scenes_d.bytes(), stream));
   ids.init(cap);
   cells.init(cell_cap);
@@ -325,6 +327,10 @@ PoolDev Group::pool() const {
   p.items = items.ptr;
   p.n_items = n_items.ptr;
   p.item_top = item_top;
+  p.units = units.ptr;
+  p.n_units = n_items.ptr + 2;
+  p.unit_top = unit_top;
+  p.vel_maps = vel_maps.ptr;
   p.tile_slot = tile_slot.ptr;
   p.slot_tile = slot_tile.ptr;
   p.tile_mark = tile_mark.ptr;
@@ -373,6 +379,8 @@ void Group::layout_changed() {
   // The work list's FP64-SVD items count down from item_top: it may change
   // only here, where a regrouping (which rebuilds the list) falls due.
   item_top = (uint32_t)items.count;
+  grow(units, max_unit_count());
+  unit_top = (uint32_t)units.count;
   if (deterministic) {
     grow(tile_item, (size_t)key_space + 2);
     grow(det_blocks, (size_t)item_top * kTileNodes);
@@ -491,6 +499,12 @@ uint32_t Group::add_scene(const mpm_config& cfg, const std::vector<mpm_rheology>
     eng->launches += 1;
   }
   MPM_CK(cudaMemsetAsync(status_d.ptr + (size_t)sid * kStatusWords, 0, kStatusWords * 4, stream));
+  if (!tile_cap && cfg.grid_size >= (uint32_t)kRegion) {
+    CUtensorMap map;
+    std::string err;
+    if (!make_velocity_map(&map, vel.ptr + g0, cfg.grid_size, &err)) throw Error(MPM_ERR_GPU, "MPM gather stage: " + err);
+    MPM_CK(cudaMemcpyAsync(vel_maps.ptr + sid, &map, sizeof(map), cudaMemcpyHostToDevice, stream));
+  }
   n_live += n;
   SceneDev d = make_scene_dev(cfg, rows, dt);
   d.n_rigid = 0;
@@ -770,7 +784,7 @@ void Group::regroup(bool compute_keys, cudaStream_t st, bool move_records) {
   // otherwise tiles cut into pieces of at most kStageMax particles, whose
   // scatter records fit the shared-memory stage.
   MPM_CK(launch_items(skeys, kCellBits, n_keep, key_space, tile_start.ptr, key_scene.ptr, scenes_d.ptr,
-                      deterministic ? 0u : item_chunk, item_top, items.ptr,
+                      deterministic ? 0u : item_chunk, item_top, items.ptr, gather_unit(), unit_top, units.ptr,
                       n_items.ptr, deterministic ? tile_item.ptr : nullptr, st));
   eng->launches += key_space ? 2 : 1;
   if (!deterministic && key_space) {
@@ -781,6 +795,13 @@ void Group::regroup(bool compute_keys, cudaStream_t st, bool move_records) {
   since = 0;
   ++regroups;
   eng->prof_end(&pr, st);
+}
+
+uint32_t Group::gather_unit() const {
+  const uint64_t warps = (uint64_t)std::max(eng->sms, 1) * std::max(occ_gather32, occ_gather64) * (kGatherThreads / 32);
+  if (n_live <= warps * kMinUnit) return kMinUnit / 2;
+  const uint64_t per = (n_live / (12 * warps) + 31) / 32 * 32;
+  return (uint32_t)std::min<uint64_t>(std::max<uint64_t>(per, kMinUnit), kMaxUnit);
 }
 
 int Group::gather_grid(bool f64) const {
@@ -807,7 +828,7 @@ void Group::launch_gather_pass(int mode, bool keys, cudaStream_t st, bool publis
   eng->prof_begin(mode == kRecord ? kStageRecord : kStageGather, st, &pr);
   for (int f64 = 0; f64 < 2; ++f64) {
     if (!(f64 ? any_svd64() : any_svd32())) continue;
-    MPM_CK(launch_gather(mode, keys, f64 != 0, pool(), f64 ? svd_tol64 : svd_tol32, svd_sweeps, reuse_svd ? 1 : 0,
+    MPM_CK(launch_gather(mode, keys, f64 != 0, pool(), f64 ? svd_tol64 : svd_tol32, svd_sweeps,
                          gather_grid(f64 != 0), st, publish_all));
     eng->launches += 1;
   }
@@ -833,7 +854,7 @@ void Group::launch_fused_pass(int acc_out, bool keys, cudaStream_t st) {
   eng->prof_begin(kStageGather, st, &pr);
   for (int f64 = 0; f64 < 2; ++f64) {
     if (!(f64 ? any_svd64() : any_svd32())) continue;
-    MPM_CK(launch_fused(keys, f64 != 0, pool(), f64 ? svd_tol64 : svd_tol32, svd_sweeps, reuse_svd ? 1 : 0, acc_out,
+    MPM_CK(launch_fused(keys, f64 != 0, pool(), f64 ? svd_tol64 : svd_tol32, svd_sweeps, acc_out,
                         fused_grid(f64 != 0), st));
     eng->launches += 1;
   }

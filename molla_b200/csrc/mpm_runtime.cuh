@@ -209,6 +209,8 @@ class Group {
   bool any_sparse() const;
   void finalize_tiles(cudaStream_t st);
   DevBuf<Item> items;
+  DevBuf<Item> units;            // the gather's cut of the same tiles (PoolDev::units)
+  DevBuf<CUtensorMap> vel_maps;  // per scene slot: tensor map of its dense velocity grid
   DevBuf<uint8_t> item_order;  // scatter lane order, 64 cells per item
   DevBuf<uint32_t> tile_item;  // deterministic mode: item of each occupied tile
   DevBuf<float4> det_blocks;   // deterministic mode: per-tile 6^3 node blocks
@@ -243,6 +245,7 @@ class Group {
   // Item slots of the work list: FP32-SVD items fill [0, n32), FP64-SVD items
   // [item_top - n64, item_top) (see k_items).
   uint32_t item_top = 0;
+  uint32_t unit_top = 0;  // the same of the gather's units
   // Scenes retired by retire_scene and not yet compacted out of the pool:
   // their particles keep their slots (the kernels skip them) until the next
   // regrouping, which sorts them behind every live particle and drops them.
@@ -250,7 +253,6 @@ class Group {
   uint32_t n_retiring = 0;    // their particles
   bool compact_issued = false;  // a regrouping that drops them was enqueued
   bool deterministic = false;
-  bool reuse_svd = true;
   double svd_tol32 = 1.0e-7;
   // Jacobi tolerance of the mixed-precision SVD, on the off-diagonal of the
   // shifted A' = F^T F - I.  F is FP32 (ulp 6e-8 near 1), so entries of A'
@@ -262,12 +264,13 @@ class Group {
   // Fused gather + scatter for the non-final substeps of the atomic P2G
   // (k_g2p2g): -1 picks it for groups of at most kFusedMaxParticles live
   // particles, 1 always, 0 never (MOLLA_MPM_FUSED=1 / 0 in the environment
-  // at construction).  Measured on a B200 with the current separate
-  // scatter: even at 133k particles, -2% at 1M, -8% at 16M, where the
-  // separate kernels' higher occupancy (4 CTAs per SM each against 2) hides
-  // the per-item barriers better than the fusion saves.
+  // at construction).  It saves a launch, which is what a small scene's
+  // substep costs (30k particles, 4 substeps with spheres: 371 us a call
+  // against 383), but holds a tile's gather in one CTA, where the separate
+  // gather spreads it over 32-particle units (133k, 20 substeps: 1.17 ms
+  // against 1.09).
   int fused_mode = -1;
-  static constexpr uint32_t kFusedMaxParticles = 262144;
+  static constexpr uint32_t kFusedMaxParticles = 65536;
   bool use_fused() const {
     // the fused kernel deposits an item before the other items are gathered,
     // so a sparse scene's tile map (built from all of them) cannot precede it
@@ -360,6 +363,16 @@ class Group {
   // a tile (the smallest item size the tuner may pick)
   static constexpr uint32_t kMinItemParticles = 128;
   size_t max_item_count() const { return (size_t)key_space + cap / kMinItemParticles + 2; }
+  // Particles per gather unit: about twelve units per resident warp, so that
+  // the list's tail is a twelfth of its time, but at least two rounds of a
+  // warp, which one fetch of the 8 KB velocity block has to serve -- or one
+  // round where two would leave warps idle.  Calls of 12..20 substeps: 133k
+  // particles 1.09 ms at 32 (1.17 at 64), 500k 6.04 at 64 (6.30 at 32, 6.47 at
+  // 128), 1M 3.92 at 64..128 (4.27 at 256), 4M 6.57 at 128 (6.63 at 96, 6.72 at
+  // 256), 16M 40.7 at 352 (41.5 at 128, 40.8 at 640).
+  static constexpr uint32_t kMinUnit = 64, kMaxUnit = 640;
+  uint32_t gather_unit() const;
+  size_t max_unit_count() const { return (size_t)key_space + cap / 32 + 2; }
   void sync_scenes(cudaStream_t st);
 
   PoolDev pool() const;

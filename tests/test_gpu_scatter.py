@@ -35,7 +35,7 @@ def test_item_sizes_match_oracle_grid(engine, n):
     sim.step(1e-4)
     gm, gp = sim.read_grid_mass_momentum()
     st = O.init_state(pts, vel, mass=cfg.particle_mass, volume=cfg.particle_volume)
-    om, op = O.step(O.make_scene(cfg, [cfg.rheology], 1e-4), st, 1)
+    om, op = O.step(O.make_scene(cfg, [cfg.rheology], 1e-4), st, 1, want_grid=True)
     total = n * cfg.particle_mass
     assert abs(gm.astype(np.float64).sum() / total - 1.0) < 1e-5
     want = (vel.astype(np.float64) * cfg.particle_mass).sum(0)
