@@ -128,8 +128,10 @@ struct mpm_sim64 {
   mpm_config cfg{};
   mpm::Scene64 sc{};
   uint32_t count = 0;
-  mpm::DevBuf<double> pos, vel, C, F, mass, vol, jp, gmass, gmom, gvel, totals;
-  mpm::DevBuf<uint32_t> mat, status;
+  mpm::DevBuf<double> pos, vel, C, F, mass, vol, jp, rec, totals;
+  mpm::DevBuf<double4> acc, gvel;
+  mpm::DevBuf<int> head, next;
+  mpm::DevBuf<uint32_t> cells, mat, status, n_cells;
 
   mpm::State64 state() {
     mpm::State64 st;
@@ -142,9 +144,13 @@ struct mpm_sim64 {
     st.vol = vol.ptr;
     st.jp = jp.ptr;
     st.mat = mat.ptr;
-    st.gmass = gmass.ptr;
-    st.gmom = gmom.ptr;
+    st.acc = acc.ptr;
     st.gvel = gvel.ptr;
+    st.rec = rec.ptr;
+    st.head = head.ptr;
+    st.next = next.ptr;
+    st.cells = cells.ptr;
+    st.n_cells = n_cells.ptr;
     st.status = status.ptr;
     return st;
   }
@@ -1707,14 +1713,16 @@ int mpm_sim64_create(mpm_engine* engine, const mpm_config* cfg, mpm_sim64** out)
     sc.sweeps = 30;
     s->set_rows(&cfg->rheology, 1);
     const size_t n3 = (size_t)sc.n * sc.n * sc.n;
-    s->gmass.alloc(n3);
-    s->gmom.alloc(3 * n3);
-    s->gvel.alloc(3 * n3);
+    REQUIRE(n3 < 0xffffffffull, MPM_ERR_INVALID, "the all-FP64 grid holds fewer than 2^32 nodes");
+    s->acc.alloc(n3);
+    s->gvel.alloc(n3);
+    s->head.alloc(n3);
+    s->n_cells.alloc(2);
     s->totals.alloc(4);
     s->status.alloc(4);
     MPM_CK(cudaMemsetAsync(s->status.ptr, 0, 16, s->eng->stream));
-    MPM_CK(cudaMemsetAsync(s->gmass.ptr, 0, n3 * 8, s->eng->stream));
-    MPM_CK(cudaMemsetAsync(s->gmom.ptr, 0, 3 * n3 * 8, s->eng->stream));
+    MPM_CK(cudaMemsetAsync(s->acc.ptr, 0, s->acc.bytes(), s->eng->stream));
+    MPM_CK(cudaMemsetAsync(s->gvel.ptr, 0, s->gvel.bytes(), s->eng->stream));
     *out = s.release();
   });
 }
@@ -1740,6 +1748,9 @@ int mpm_sim64_set_particles(mpm_sim64* sim, const double* xyz, uint32_t n) {
     sim->vol.alloc(m);
     sim->jp.alloc(m);
     sim->mat.alloc(m);
+    sim->rec.alloc(16 * m);
+    sim->next.alloc(m);
+    sim->cells.alloc(m);
     std::vector<double> F(9 * m, 0.0), mass(m, (double)sim->cfg.particle_mass), vol(m, (double)sim->cfg.particle_volume);
     for (size_t i = 0; i < m; ++i) F[9 * i] = F[9 * i + 4] = F[9 * i + 8] = 1.0;
     cudaStream_t st = sim->eng->stream;
@@ -1778,8 +1789,7 @@ int mpm_sim64_step_n(mpm_sim64* sim, double dt, uint32_t substeps) {
     sim->eng->check();
     sim->sc.dt = dt;
     sim->sc.gy = (double)sim->cfg.gravity_y;
-    MPM_CK(mpm::launch_step64(sim->sc, sim->state(), substeps, sim->eng->stream));
-    sim->eng->launches += (uint64_t)substeps * 4;
+    MPM_CK(mpm::launch_step64(sim->sc, sim->state(), substeps, sim->eng->stream, &sim->eng->launches));
   });
 }
 
