@@ -39,9 +39,11 @@ __device__ __forceinline__ uint32_t tile_key_of(const SceneDev& sc, float x, flo
 
 }  // namespace
 
-// grid_update (mpm.wgsl:1013-1058) over the grid pool, kGridBlocksPerCta
-// 256-cell pool blocks per thread block, one node of each per thread
-// (grid_node is the per-node body).  Only blocks the last scatter touched
+// grid_update (mpm.wgsl:1013-1058) over the grid pool, `per_cta` 256-cell pool
+// blocks per thread block (grid_node is the per-node body): one warp reads
+// their marks and lists those with work, and the thread block then takes the
+// listed ones four at a time, one node of each per thread, with their loads in
+// flight together.  Only blocks the last scatter touched
 // (or a rigid sphere may reach) are converted; the blocks touched by the scatter before it are
 // cleared in the other accumulator (ready for the next scatter) and
 // unmarked.  Counts completed substeps.  The rigid-sphere imprint
@@ -50,7 +52,17 @@ __device__ __forceinline__ uint32_t tile_key_of(const SceneDev& sc, float x, flo
 // 1e6, its sand mass and momentum give the reaction wrench, and the node is
 // marked rigid (negative w in the velocity buffer) so that gravity, walls
 // and the implicit sweeps leave it alone.
-constexpr int kGridBlocksPerCta = 4;
+constexpr int kGridTogether = 4;
+// Pool blocks per thread block: four while that fills the chip (a 64^3 grid
+// has 1,024 in all), up to 32 where most blocks are idle and reading their
+// marks a few bytes per thread block is what costs (a 256^3 grid with 13% of
+// its blocks touched: 90 -> 56 us; sparse storage of 65,536 tiles, 1,450 of them
+// active: 37 us -> under 10).
+constexpr int kGridMaxPerCta = 32;
+inline int grid_blocks_per_cta(uint64_t pool_blocks) {
+  const uint64_t want = pool_blocks / (148 * 4) / kGridTogether * kGridTogether;
+  return (int)std::min<uint64_t>(std::max<uint64_t>(want, kGridTogether), kGridMaxPerCta);
+}
 
 __device__ __forceinline__ void grid_node(const PoolDev& p, uint32_t sid, const SceneDev& sc, uint64_t blk,
                                           uint64_t g, float4 a, bool in_a, bool rb, int acc_in) {
@@ -128,60 +140,75 @@ __device__ __forceinline__ void grid_node(const PoolDev& p, uint32_t sid, const 
   p.vel[g] = make_float4(v[0], v[1], v[2], m);
 }
 
-__global__ void __launch_bounds__(kCellThreads, 5) k_grid_update(PoolDev p, const uint32_t* __restrict__ block_scene,
-                                                              uint64_t total_cells, int acc_in, int count_substep) {
+__global__ void __launch_bounds__(kCellThreads, 4) k_grid_update(PoolDev p, const uint32_t* __restrict__ block_scene,
+                                                              uint64_t total_cells, int per_cta, int acc_in,
+                                                              int count_substep) {
   static_assert(kCellThreads == kCellBlock, "one thread per cell of a grid-pool block");
-  constexpr int K = kGridBlocksPerCta;
+  static_assert(kGridMaxPerCta == 32, "one lane per pool block");
+  struct Work {
+    uint32_t blk, sid, valid;  // pool block, its scene, its nodes that belong to the grid (0..256)
+    uint32_t flags;            // 1: convert, 2: clear the other accumulator, 4: a rigid sphere may reach it, 8: deposits
+  };
+  __shared__ Work s_work[kGridMaxPerCta];
+  __shared__ uint32_t s_n;
   launch_next();
   wait_previous();
   if (blockIdx.x == 0 && threadIdx.x < (unsigned)kWorkWords) p.work[threadIdx.x] = 0u;
-  // Every load of the marks and of the accumulators is issued before any is
-  // used, so that a thread keeps K requests in flight.
-  uint32_t sid[K];
-  bool in_a[K], in_b[K], rb[K], conv[K];
-  float4 acc_v[K];
-#pragma unroll
-  for (int b = 0; b < K; ++b) {
-    const uint64_t blk = (uint64_t)blockIdx.x * K + b;
-    const bool exists = blk * kCellThreads < total_cells;
-    sid[b] = exists ? block_scene[blk] : 0xffffffffu;
-    in_a[b] = exists && p.touched[acc_in][blk] != 0;
-    in_b[b] = exists && p.touched[acc_in ^ 1][blk] != 0;
-    rb[b] = exists && p.rigid_blocks[blk] != 0;
-  }
-#pragma unroll
-  for (int b = 0; b < K; ++b) {
-    conv[b] = false;
-    if (sid[b] == 0xffffffffu) continue;
-    const uint64_t g = ((uint64_t)blockIdx.x * K + b) * kCellThreads + threadIdx.x;
-    if (in_b[b]) p.acc[acc_in ^ 1][g] = make_float4(0.f, 0.f, 0.f, 0.f);
-    const SceneDev& sc = p.scenes[sid[b]];
-    const uint64_t local64 = g - sc.grid_off;
-    if (count_substep && local64 == 0) {
-      // completed substeps; a scene with a budget counts one past it and
-      // stops there (its particle kernels then stand still)
+  if (threadIdx.x < 32) {
+    const uint64_t blk = (uint64_t)blockIdx.x * per_cta + threadIdx.x;
+    const bool exists = (int)threadIdx.x < per_cta && blk * kCellThreads < total_cells;
+    Work wk{(uint32_t)blk, exists ? block_scene[blk] : 0xffffffffu, 0u, 0u};
+    const bool in_a = exists && p.touched[acc_in][blk] != 0;
+    const bool in_b = exists && p.touched[acc_in ^ 1][blk] != 0;
+    const bool rb = exists && p.rigid_blocks[blk] != 0;
+    if (wk.sid != 0xffffffffu) {
+      const SceneDev& sc = p.scenes[wk.sid];
+      const uint64_t local = blk * kCellThreads - sc.grid_off;
       volatile uint32_t* status = p.status + (size_t)sc.status * kStatusWords;
-      if (status[0] == 0u && (status[2] == 0u || status[1] <= status[2]))
-        atomicAdd(const_cast<uint32_t*>(status) + 1, 1u);
+      if (count_substep && local == 0) {
+        // completed substeps; a scene with a budget counts one past it and
+        // stops there (its particle kernels then stand still)
+        if (status[0] == 0u && (status[2] == 0u || status[1] <= status[2]))
+          atomicAdd(const_cast<uint32_t*>(status) + 1, 1u);
+      }
+      if (in_a || rb) {
+        // dense: the n^3 block; sparse: the slots of the current tile map
+        const uint64_t extent = sc.tile_cap ? 64ull * min(status[3], sc.tile_cap) : (uint64_t)sc.n * sc.n * sc.n;
+        wk.valid = extent > local ? (uint32_t)min(extent - local, (uint64_t)kCellThreads) : 0u;
+        if (wk.valid) wk.flags = 1u | (rb ? 4u : 0u) | (in_a ? 8u : 0u);
+      }
+      if (in_b) {
+        wk.flags |= 2u;
+        p.touched[acc_in ^ 1][blk] = 0;  // read by no other thread block
+      }
     }
-    // dense: the n^3 block; sparse: the slots of the current tile map
-    const uint64_t extent =
-        sc.tile_cap ? 64ull * min(*((volatile uint32_t*)p.status + (size_t)sc.status * kStatusWords + 3), sc.tile_cap)
-                    : (uint64_t)sc.n * sc.n * sc.n;
-    conv[b] = (in_a[b] || rb[b]) && local64 < extent;
-    if (conv[b]) acc_v[b] = p.acc[acc_in][g];
+    const uint32_t list = __ballot_sync(0xffffffffu, wk.flags != 0u);
+    if (wk.flags) s_work[__popc(list & ((1u << threadIdx.x) - 1u))] = wk;
+    if (threadIdx.x == 0) s_n = __popc(list);
   }
-  __syncthreads();  // every thread has read the marks
-  if (threadIdx.x == 0) {
+  __syncthreads();
+  const uint32_t n = s_n;
+  for (uint32_t e = 0; e < n; e += kGridTogether) {
+    // every accumulator load is issued before any is used
+    bool conv[kGridTogether];
+    float4 acc_v[kGridTogether];
 #pragma unroll
-    for (int b = 0; b < K; ++b)
-      if (sid[b] != 0xffffffffu && in_b[b]) p.touched[acc_in ^ 1][(uint64_t)blockIdx.x * K + b] = 0;
-  }
+    for (int b = 0; b < kGridTogether; ++b) {
+      conv[b] = false;
+      if (e + b >= n) continue;
+      const Work wk = s_work[e + b];
+      const uint64_t g = (uint64_t)wk.blk * kCellThreads + threadIdx.x;
+      if (wk.flags & 2u) p.acc[acc_in ^ 1][g] = make_float4(0.f, 0.f, 0.f, 0.f);
+      conv[b] = (wk.flags & 1u) && threadIdx.x < wk.valid;
+      if (conv[b]) acc_v[b] = p.acc[acc_in][g];
+    }
 #pragma unroll
-  for (int b = 0; b < K; ++b) {
-    if (!conv[b]) continue;
-    const uint64_t blk = (uint64_t)blockIdx.x * K + b;
-    grid_node(p, sid[b], p.scenes[sid[b]], blk, blk * kCellThreads + threadIdx.x, acc_v[b], in_a[b], rb[b], acc_in);
+    for (int b = 0; b < kGridTogether; ++b) {
+      if (!conv[b]) continue;
+      const Work wk = s_work[e + b];
+      grid_node(p, wk.sid, p.scenes[wk.sid], wk.blk, (uint64_t)wk.blk * kCellThreads + threadIdx.x, acc_v[b],
+                (wk.flags & 8u) != 0, (wk.flags & 4u) != 0, acc_in);
+    }
   }
 }
 
@@ -191,6 +218,8 @@ __global__ void __launch_bounds__(kCellThreads, 5) k_grid_update(PoolDev p, cons
 // and its torque to the sphere's wrench.
 __global__ void __launch_bounds__(kCellThreads) k_rigid_shell(PoolDev p, const uint32_t* __restrict__ block_scene,
                                                               uint64_t total_cells, int acc_in) {
+  launch_next();
+  wait_previous();
   const uint64_t blk = blockIdx.x;
   if (blk * kCellThreads >= total_cells) return;
   const uint32_t sid = block_scene[blk];
@@ -240,6 +269,8 @@ __global__ void __launch_bounds__(kCellThreads) k_grid_jacobi(PoolDev p, const u
                                                               uint64_t total_cells, int acc_in,
                                                               const float4* __restrict__ src, float4* __restrict__ dst,
                                                               uint32_t sweep) {
+  launch_next();
+  wait_previous();
   const uint64_t blk = blockIdx.x;
   if (blk * kCellThreads >= total_cells) return;
   const uint32_t sid = block_scene[blk];
@@ -290,19 +321,6 @@ __global__ void __launch_bounds__(kCellThreads) k_grid_jacobi(PoolDev p, const u
               vz = (m * cur.z + alpha * az) / denom;
   const bool nan = !(vx == vx) || !(vy == vy) || !(vz == vz);
   dst[g] = nan ? make_float4(cur.x, cur.y, cur.z, m) : make_float4(vx, vy, vz, m);
-}
-
-// dst <- src over the touched blocks (the last Jacobi sweep's result back into
-// the velocity buffer the gather reads).
-__global__ void __launch_bounds__(kCellThreads) k_vel_copy(const uint8_t* __restrict__ touched,
-                                                           const uint32_t* __restrict__ block_scene,
-                                                           uint64_t total_cells, const float4* __restrict__ src,
-                                                           float4* __restrict__ dst) {
-  const uint64_t blk = blockIdx.x;
-  if (blk * kCellThreads >= total_cells) return;
-  if (block_scene[blk] == 0xffffffffu || !touched[blk]) return;
-  const uint64_t g = blk * kCellThreads + threadIdx.x;
-  dst[g] = src[g];
 }
 
 // Sort keys of the live slots (tile_keys, mpm_particle_order.wgsl:11-25)
@@ -389,6 +407,8 @@ __global__ void k_reorder(const float* __restrict__ src, float* __restrict__ dst
                           const uint32_t* __restrict__ ids, const uint32_t* __restrict__ keys,
                           uint32_t* __restrict__ slot_key, const float4* __restrict__ rec_src,
                           float4* __restrict__ rec_dst, uint32_t n_live) {
+  launch_next();
+  wait_previous();
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n_live) return;
   const uint32_t id = ids[s];
@@ -405,18 +425,15 @@ __global__ void k_reorder(const float* __restrict__ src, float* __restrict__ dst
   slot_of[id] = s;
 }
 
-// tile_start[t] = first sorted position whose key is >= t, for t in [0, K].
-__global__ void k_tile_start(const uint32_t* __restrict__ sorted_keys, uint32_t n_live, uint32_t K, int shift,
-                             uint32_t* __restrict__ tile_start) {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t > K) return;
-  uint32_t lo = 0, hi = n_live;
+// First position in [lo, hi) of the sorted keys whose tile (key >> shift) is >= t, or hi.
+__device__ __forceinline__ uint32_t tile_lower(const uint32_t* __restrict__ sorted_keys, uint32_t lo, uint32_t hi,
+                                               int shift, uint32_t t) {
   while (lo < hi) {
     const uint32_t mid = lo + (hi - lo) / 2;
     if ((sorted_keys[mid] >> shift) < t) lo = mid + 1;
     else hi = mid;
   }
-  tile_start[t] = lo;
+  return lo;
 }
 
 // Work items: every occupied tile, cut into chunks of at most `chunk` slots.
@@ -427,14 +444,16 @@ __global__ void k_tile_start(const uint32_t* __restrict__ sorted_keys, uint32_t 
 // a contiguous range.  The gather's units are cut from the same tiles in the
 // same way (counts n_items[2], n_items[3]), into equal pieces of whole rounds
 // of a warp and at most about `unit` slots.
-__global__ void k_items(const uint32_t* __restrict__ tile_start, uint32_t K, const uint32_t* __restrict__ key_scene,
+__global__ void k_items(const uint32_t* __restrict__ sorted_keys, uint32_t n_live, int shift, uint32_t K,
+                        const uint32_t* __restrict__ key_scene,
                         const SceneDev* __restrict__ scenes, uint32_t chunk, uint32_t item_top,
                         Item* __restrict__ items, uint32_t unit, uint32_t unit_top, Item* __restrict__ units,
                         uint32_t* __restrict__ n_items, uint32_t* __restrict__ tile_item) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= K) return;
-  const uint32_t a = tile_start[t], b = tile_start[t + 1];
-  if (b <= a) return;
+  const uint32_t a = tile_lower(sorted_keys, 0u, n_live, shift, t);
+  if (a >= n_live || (sorted_keys[a] >> shift) != t) return;
+  const uint32_t b = tile_lower(sorted_keys, a, n_live, shift, t + 1u);
   const uint32_t scene = key_scene[t];
   if (scene == 0xffffffffu) return;  // no live scene holds this key (cannot carry particles)
   const uint32_t cnt = b - a;
@@ -545,6 +564,8 @@ __global__ void __launch_bounds__(64) k_item_order(const Item* __restrict__ item
   __shared__ uint32_t s_cnt[64];
   __shared__ uint8_t s_pair[32][2];
   __shared__ uint32_t s_fill[32];
+  launch_next();
+  wait_previous();
   const uint32_t n32 = n_items[0], total = n32 + n_items[1];
   for (uint32_t li = blockIdx.x; li < total; li += gridDim.x) {
     const uint32_t it = li < n32 ? li : item_top - 1u - (li - n32);
@@ -632,34 +653,25 @@ __global__ void k_totals(PoolDev p, int acc_idx, uint64_t grid_off, uint64_t cel
 cudaError_t launch_grid_update(const PoolDev& p, const uint32_t* block_scene, uint64_t total_cells, int acc_in,
                                int count_substep, cudaStream_t st) {
   const uint64_t pool_blocks = (total_cells + kCellThreads - 1) / kCellThreads;
-  const uint64_t blocks = (pool_blocks + kGridBlocksPerCta - 1) / kGridBlocksPerCta;
-  if (blocks == 0) return cudaSuccess;
-  return launch_dependent(k_grid_update, (int)blocks, kCellThreads, 0, st, p, block_scene, total_cells, acc_in,
-                          count_substep);
+  if (pool_blocks == 0) return cudaSuccess;
+  const int per_cta = grid_blocks_per_cta(pool_blocks);
+  return launch_dependent(k_grid_update, (int)((pool_blocks + per_cta - 1) / per_cta), kCellThreads, 0, st, p,
+                          block_scene, total_cells, per_cta, acc_in, count_substep);
 }
 
 cudaError_t launch_grid_jacobi(const PoolDev& p, const uint32_t* block_scene, uint64_t total_cells, int acc_in,
                                const float4* src, float4* dst, uint32_t sweep, cudaStream_t st) {
   const uint64_t blocks = (total_cells + kCellThreads - 1) / kCellThreads;
   if (blocks == 0) return cudaSuccess;
-  k_grid_jacobi<<<(unsigned)blocks, kCellThreads, 0, st>>>(p, block_scene, total_cells, acc_in, src, dst, sweep);
-  return cudaGetLastError();
+  return launch_dependent(k_grid_jacobi, (int)blocks, kCellThreads, 0, st, p, block_scene, total_cells, acc_in, src, dst,
+                          sweep);
 }
 
 cudaError_t launch_rigid_shell(const PoolDev& p, const uint32_t* block_scene, uint64_t total_cells, int acc_in,
                                cudaStream_t st) {
   const uint64_t blocks = (total_cells + kCellThreads - 1) / kCellThreads;
   if (blocks == 0) return cudaSuccess;
-  k_rigid_shell<<<(unsigned)blocks, kCellThreads, 0, st>>>(p, block_scene, total_cells, acc_in);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_vel_copy(const uint8_t* touched, const uint32_t* block_scene, uint64_t total_cells,
-                            const float4* src, float4* dst, cudaStream_t st) {
-  const uint64_t blocks = (total_cells + kCellThreads - 1) / kCellThreads;
-  if (blocks == 0) return cudaSuccess;
-  k_vel_copy<<<(unsigned)blocks, kCellThreads, 0, st>>>(touched, block_scene, total_cells, src, dst);
-  return cudaGetLastError();
+  return launch_dependent(k_rigid_shell, (int)blocks, kCellThreads, 0, st, p, block_scene, total_cells, acc_in);
 }
 
 cudaError_t launch_keys(const PoolDev& p, uint32_t n_slots, cudaStream_t st) {
@@ -696,20 +708,18 @@ cudaError_t launch_reorder(const float* src, float* dst, uint32_t cap, const uin
                            uint32_t* slot_key, const float4* rec_src, float4* rec_dst, uint32_t n_live,
                            cudaStream_t st) {
   if (!n_live) return cudaSuccess;
-  k_reorder<<<(n_live + 255) / 256, 256, 0, st>>>(src, dst, cap, meta_src, meta_dst, orig_dst, slot_of, ids, keys,
-                                                  slot_key, rec_src, rec_dst, n_live);
-  return cudaGetLastError();
+  return launch_dependent(k_reorder, (int)((n_live + 255) / 256), 256, 0, st, src, dst, cap, meta_src, meta_dst, orig_dst,
+                          slot_of, ids, keys, slot_key, rec_src, rec_dst, n_live);
 }
 
-cudaError_t launch_items(const uint32_t* sorted_keys, int shift, uint32_t n_live, uint32_t K, uint32_t* tile_start,
+cudaError_t launch_items(const uint32_t* sorted_keys, int shift, uint32_t n_live, uint32_t K,
                          const uint32_t* key_scene, const SceneDev* scenes, uint32_t chunk, uint32_t item_top,
                          Item* items, uint32_t unit, uint32_t unit_top, Item* units, uint32_t* n_items,
                          uint32_t* tile_item, cudaStream_t st) {
   cudaMemsetAsync(n_items, 0, 4 * sizeof(uint32_t), st);
   if (tile_item) cudaMemsetAsync(tile_item, 0xff, (size_t)(K + 1) * sizeof(uint32_t), st);
-  k_tile_start<<<(K + 1 + 255) / 256, 256, 0, st>>>(sorted_keys, n_live, K, shift, tile_start);
   if (K > 0)
-    k_items<<<(K + 255) / 256, 256, 0, st>>>(tile_start, K, key_scene, scenes, chunk, item_top, items, unit, unit_top,
+    k_items<<<(K + 255) / 256, 256, 0, st>>>(sorted_keys, n_live, shift, K, key_scene, scenes, chunk, item_top, items, unit, unit_top,
                                              units, n_items, tile_item);
   return cudaGetLastError();
 }
@@ -718,6 +728,8 @@ cudaError_t launch_items(const uint32_t* sorted_keys, int shift, uint32_t n_live
 // hashed map every step, crates/molla-solvers/src/mpm_active_tiles.rs:242-302):
 // the active-tile counters of the sparse scenes start at zero ...
 __global__ void k_tiles_reset(PoolDev p, uint32_t n_scenes) {
+  launch_next();
+  wait_previous();
   for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < n_scenes; s += gridDim.x * blockDim.x) {
     const SceneDev& sc = p.scenes[s];
     if (sc.live && sc.tile_cap) p.status[(size_t)sc.status * kStatusWords + 3] = 0u;
@@ -730,6 +742,8 @@ __global__ void k_tiles_reset(PoolDev p, uint32_t n_scenes) {
 // kFaultTileOverflow; the excess tiles get no slot (their deposits are
 // dropped and the scene freezes from the next substep).
 __global__ void k_tiles_finalize(PoolDev p, const uint32_t* __restrict__ key_scene, uint32_t K) {
+  launch_next();
+  wait_previous();
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= K) return;
   const uint32_t sid = key_scene[t];
@@ -753,9 +767,9 @@ __global__ void k_tiles_finalize(PoolDev p, const uint32_t* __restrict__ key_sce
 
 cudaError_t launch_tiles_finalize(const PoolDev& p, const uint32_t* key_scene, uint32_t K, uint32_t n_scenes,
                                   cudaStream_t st) {
-  k_tiles_reset<<<(n_scenes + 255) / 256, 256, 0, st>>>(p, n_scenes);
-  if (K) k_tiles_finalize<<<(K + 255) / 256, 256, 0, st>>>(p, key_scene, K);
-  return cudaGetLastError();
+  const cudaError_t e = launch_dependent(k_tiles_reset, (int)((n_scenes + 255) / 256), 256, 0, st, p, n_scenes);
+  if (e != cudaSuccess || !K) return e;
+  return launch_dependent(k_tiles_finalize, (int)((K + 255) / 256), 256, 0, st, p, key_scene, K);
 }
 
 __global__ void k_fill_u32(uint32_t* __restrict__ p, uint64_t n, uint32_t v) {
@@ -773,9 +787,8 @@ cudaError_t launch_fill_u32(uint32_t* p, uint64_t n, uint32_t v, cudaStream_t st
 cudaError_t launch_item_order(const Item* items, const uint32_t* n_items, uint32_t item_top, const uint32_t* slot_key,
                               uint8_t* item_order, cudaStream_t st) {
   if (!item_top) return cudaSuccess;
-  k_item_order<<<std::min<uint32_t>(item_top, 148u * 32u), 64, 0, st>>>(items, n_items, item_top, slot_key,
-                                                                        item_order);
-  return cudaGetLastError();
+  return launch_dependent(k_item_order, (int)std::min<uint32_t>(item_top, 148u * 32u), 64, 0, st, items, n_items, item_top,
+                          slot_key, item_order);
 }
 
 cudaError_t launch_gather_xyz(const PoolDev& p, int first, const uint32_t* slot_of, uint32_t id_base, uint32_t n,

@@ -97,11 +97,9 @@ cudaError_t launch_grid_jacobi(const PoolDev& p, const uint32_t* block_scene, ui
 // Rigid-sphere shell reaction over the touched blocks a sphere may reach.
 cudaError_t launch_rigid_shell(const PoolDev& p, const uint32_t* block_scene, uint64_t total_cells, int acc_in,
                                cudaStream_t st);
-cudaError_t launch_vel_copy(const uint8_t* touched, const uint32_t* block_scene, uint64_t total_cells,
-                            const float4* src, float4* dst, cudaStream_t st);
 // Work list of the regrouped particles (see k_items): FP32-SVD items in slots
 // [0, n_items[0]), FP64-SVD items in [item_top - n_items[1], item_top).
-cudaError_t launch_items(const uint32_t* sorted_keys, int shift, uint32_t n_live, uint32_t K, uint32_t* tile_start,
+cudaError_t launch_items(const uint32_t* sorted_keys, int shift, uint32_t n_live, uint32_t K,
                          const uint32_t* key_scene, const SceneDev* scenes, uint32_t chunk, uint32_t item_top,
                          Item* items, uint32_t unit, uint32_t unit_top, Item* units, uint32_t* n_items,
                          uint32_t* tile_item, cudaStream_t st);

@@ -370,7 +370,6 @@ template <class T> static void grow_keep(DevBuf<T>& b, size_t need, cudaStream_t
 
 void Group::layout_changed() {
   key_space = (uint32_t)keyr.high_water();
-  grow(tile_start, (size_t)key_space + 2);
   const size_t max_items = max_item_count();
   if (items.count < max_items) {
     grow(items, max_items);
@@ -783,10 +782,10 @@ void Group::regroup(bool compute_keys, cudaStream_t st, bool move_records) {
   // Items: whole tiles for the fixed-order scatter (one item per tile);
   // otherwise tiles cut into pieces of at most kStageMax particles, whose
   // scatter records fit the shared-memory stage.
-  MPM_CK(launch_items(skeys, kCellBits, n_keep, key_space, tile_start.ptr, key_scene.ptr, scenes_d.ptr,
+  MPM_CK(launch_items(skeys, kCellBits, n_keep, key_space, key_scene.ptr, scenes_d.ptr,
                       deterministic ? 0u : item_chunk, item_top, items.ptr, gather_unit(), unit_top, units.ptr,
                       n_items.ptr, deterministic ? tile_item.ptr : nullptr, st));
-  eng->launches += key_space ? 2 : 1;
+  eng->launches += key_space ? 1 : 0;
   if (!deterministic && key_space) {
     MPM_CK(launch_item_order(items.ptr, n_items.ptr, item_top, slot_key.ptr, item_order.ptr, st));
     eng->launches += 1;
@@ -1068,26 +1067,21 @@ uint32_t Group::max_jacobi_iters() const {
 void Group::grid_pass(int a, uint32_t max_jacobi, bool rigid, cudaStream_t st) {
   const uint64_t total_cells = cells.high_water();
   if (rigid) MPM_CK(cudaMemsetAsync(wrench_d.ptr, 0, wrench_d.bytes(), st));  // wrench of this substep only
-  MPM_CK(launch_grid_update(pool(), block_scene.ptr, total_cells, a, 1, st));
-  eng->launches += 1;
-  if (max_jacobi) jacobi_pass(a, max_jacobi, st);
-  if (rigid) {
-    MPM_CK(launch_rigid_shell(pool(), block_scene.ptr, total_cells, a, st));
-    eng->launches += 1;
-  }
-}
-
-void Group::jacobi_pass(int a, uint32_t max_jacobi, cudaStream_t st) {
-  const uint64_t total_cells = cells.high_water();
+  // The sweeps ping-pong between two buffers; the grid update writes the one
+  // from which their last lands in the buffer the gather reads.
   float4* bufs[2] = {vel.ptr, vel2.ptr};
-  int cur = 0;
+  int cur = (int)(max_jacobi & 1u);
+  PoolDev p = pool();
+  p.vel = bufs[cur];
+  MPM_CK(launch_grid_update(p, block_scene.ptr, total_cells, a, 1, st));
+  eng->launches += 1;
   for (uint32_t k = 0; k < max_jacobi; ++k) {
     MPM_CK(launch_grid_jacobi(pool(), block_scene.ptr, total_cells, a, bufs[cur], bufs[cur ^ 1], k, st));
     eng->launches += 1;
     cur ^= 1;
   }
-  if (cur) {
-    MPM_CK(launch_vel_copy(touched[a].ptr, block_scene.ptr, total_cells, bufs[1], bufs[0], st));
+  if (rigid) {
+    MPM_CK(launch_rigid_shell(pool(), block_scene.ptr, total_cells, a, st));
     eng->launches += 1;
   }
 }

@@ -195,7 +195,7 @@ class Group {
   // scenes
   DevBuf<SceneDev> scenes_d;
   DevBuf<uint32_t> status_d;
-  DevBuf<uint32_t> tile_start, n_items;
+  DevBuf<uint32_t> n_items;
   // Scene of every tile key (0xffffffff: no live scene).  Each scene holds a
   // stable range of the key space (allocated from `keyr` when it is added),
   // so adding or retiring a scene re-keys no other scene.
@@ -357,7 +357,6 @@ class Group {
   // Grid update of accumulator a, then the semi-implicit Jacobi sweeps of
   // the scenes that ask for them.
   void grid_pass(int a, uint32_t max_jacobi, bool rigid, cudaStream_t st);
-  void jacobi_pass(int a, uint32_t max_jacobi, cudaStream_t st);
   uint32_t max_jacobi_iters() const;
   // one item per occupied tile, plus one per kMinItemParticles particles of
   // a tile (the smallest item size the tuner may pick)
