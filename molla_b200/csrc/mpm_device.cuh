@@ -128,7 +128,9 @@ struct PoolDev {
   const RigidDev* rigid;        // kMaxRigid per scene
   float* wrench;                // 8 floats per sphere slot: force xyz, 0, torque xyz, 0
   float4* vel;          // grid velocity (vx, vy, vz, mass)
-  float* rec;           // per slot 16 floats, the deposit form (see make_record): (m, q), (Bd0..3), (Bd4..7), (Bd8, xp)
+  // per slot 16 floats, in the deposit's form (particle_step): (m, q), (Bd0..3), (Bd4..7), (Bd8, xp); in the
+  // fixed-order mode (x, y, z, m), (m v, B0), (B1..B4), (B5..B8)
+  float* rec;
   const uint32_t* slot_key;  // regroup key of each slot: (tile << 6) | cell in tile
   const SceneDev* scenes;
   uint32_t* status;     // kStatusWords per scene
@@ -200,25 +202,33 @@ __device__ __forceinline__ int64_t node_index(const SC& sc, const uint32_t* __re
 }
 
 // Marks the tiles of the 3^3 stencil of a particle with base node (bx, by,
-// bz) in a sparse scene (1 or 2 tiles per axis).
-__device__ __forceinline__ void mark_stencil_tiles(const SceneDev& sc, uint8_t* __restrict__ tile_mark, int bx, int by,
-                                                   int bz) {
+// bz) in a sparse scene (1 or 2 tiles per axis).  For particles that left the
+// block of their unit's tile; the others' tiles are gathered per unit.
+static __device__ __noinline__ void mark_far_tiles(const SceneDev& sc, uint8_t* __restrict__ tile_mark, int bx, int by, int bz) {
   const int n = (int)sc.n;
-  int lo[3], hi[3];
   const int b[3] = {bx, by, bz};
-#pragma unroll
+  int lo[3], hi[3];
   for (int a = 0; a < 3; ++a) {
     const int l = max(b[a], 0), h = min(b[a] + 2, n - 1);
     if (l > h) return;  // the stencil misses the grid on this axis
     lo[a] = l >> 2;
     hi[a] = h >> 2;
   }
-  for (int tz = lo[2]; tz <= hi[2]; ++tz)
-    for (int ty = lo[1]; ty <= hi[1]; ++ty)
-      for (int tx = lo[0]; tx <= hi[0]; ++tx) {
-        uint8_t* m = tile_mark + sc.key_off + (uint32_t)tx + sc.w * ((uint32_t)ty + sc.w * (uint32_t)tz);
-        if (*m == 0) *m = 1;
-      }
+#pragma unroll 1
+  for (int q = 0; q < 8; ++q) {
+    const int tx = (q & 1) ? hi[0] : lo[0], ty = (q & 2) ? hi[1] : lo[1], tz = (q & 4) ? hi[2] : lo[2];
+    tile_mark[sc.key_off + (uint32_t)tx + sc.w * ((uint32_t)ty + sc.w * (uint32_t)tz)] = 1;
+  }
+}
+
+// The tiles (of the 27 around the unit's own, bit (dx + 1) + 3 (dy + 1) + 9 (dz +
+// 1)) that the stencil of base node l of the unit's 8^3 block touches, 0 <= l <=
+// 5: region coordinate r lies in tile (r + 3) / 4 - 1 on its axis.
+__device__ __forceinline__ uint32_t block_tiles(int lx, int ly, int lz) {
+  const uint32_t x = (1u << ((lx + 3) >> 2)) | (1u << ((lx + 5) >> 2));
+  const uint32_t y = (1u << (3 * ((ly + 3) >> 2))) | (1u << (3 * ((ly + 5) >> 2)));
+  const uint32_t z = (1u << (9 * ((lz + 3) >> 2))) | (1u << (9 * ((lz + 5) >> 2)));
+  return x * y * z;  // the set bits of x, y and z lie in different digits: no two products meet
 }
 
 // Whether a scene's particles stand still this substep: a latched fault, or
@@ -282,6 +292,15 @@ __device__ __forceinline__ void matmul(const T* a, const T* b, T* o) {
 #pragma unroll
     for (int r = 0; r < 3; ++r) o[3 * c + r] = a[r] * b[3 * c] + a[3 + r] * b[3 * c + 1] + a[6 + r] * b[3 * c + 2];
 }
+// u * diag(d) * v^T
+template <class T>
+__device__ __forceinline__ void sandwich(const T* u, const T* d, const T* v, T* o) {
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+      o[3 * c + r] = (u[r] * d[0]) * v[c] + (u[3 + r] * d[1]) * v[3 + c] + (u[6 + r] * d[2]) * v[6 + c];
+}
 template <class T>
 __device__ __forceinline__ T det3(const T* a) {
   // first-column expansion; a[3*col+row]
@@ -310,11 +329,7 @@ __device__ __forceinline__ T det3(const T* a) {
 // the stress record and F's update, are FP32); sigma carries the form's
 // precision.
 //
-// FP32 form: sigma_i = |F v_i| and u_i = F v_i / sigma_i in FP32 (hardware
-// reciprocal square root and one Newton step), and e_i = sigma_i - 1 from the
-// eigenvalue of A' where F is near a rotation: lambda'_i = sigma_i^2 - 1, so
-// e_i = lambda'_i / (1 + sigma_i) keeps the relative precision of A' where
-// sigma_i - 1 would keep only the half ulp of 1 that sigma_i was rounded to.
+// FP32 form: sigma_i = |F v_i| and u_i = F v_i / sigma_i in FP32.
 //
 // FP64 form (svd3<double>): sigma_i = |F v_i| / |v_i| in FP64.  Double
 // division and square roots are replaced by Newton-Raphson refinement of
@@ -323,7 +338,6 @@ __device__ __forceinline__ T det3(const T* a) {
 template <class T> struct SvdOut {
   float u[9], v[9];
   T s[3];
-  float e[3];  // sigma - 1 (FP32 form only)
 };
 
 // Newton-Raphson reciprocal square root of x > 0: y <- y (3 - x y^2) / 2
@@ -446,17 +460,18 @@ __device__ __forceinline__ void svd3(const T* f, const float* f32, SvdOut<T>& o,
       const float y = f[1] * v[3 * i] + f[4] * v[3 * i + 1] + f[7] * v[3 * i + 2];
       const float z = f[2] * v[3 * i] + f[5] * v[3 * i + 1] + f[8] * v[3 * i + 2];
       const float q = x * x + y * y + z * z;
-      // sqrt(q) and its reciprocal by one Newton step each; q = NaN or
-      // infinite gives NaN, which the caller's check of sigma finds
-      const float r = rsqrtf(q);
-      float s = q * r;
-      s = fmaf(fmaf(-s, s, q), 0.5f * r, s);
-      const bool zero = q <= 1.0e-24f;
-      o.s[i] = zero ? 0.0f : s;
-      const float inv = r * fmaf(-0.5f * q * r, r, 1.5f);
-      o.u[3 * i] = zero ? (i == 0 ? 1.0f : 0.0f) : x * inv;
-      o.u[3 * i + 1] = zero ? (i == 1 ? 1.0f : 0.0f) : y * inv;
-      o.u[3 * i + 2] = zero ? (i == 2 ? 1.0f : 0.0f) : z * inv;
+      const float s = sqrtf(q);  // correctly rounded: the stress depends on s - 1
+      o.s[i] = s;
+      if (s > 1.0e-12f) {
+        const float inv = __frcp_rn(s);
+        o.u[3 * i] = x * inv;
+        o.u[3 * i + 1] = y * inv;
+        o.u[3 * i + 2] = z * inv;
+      } else {
+        o.u[3 * i] = i == 0 ? 1.0f : 0.0f;
+        o.u[3 * i + 1] = i == 1 ? 1.0f : 0.0f;
+        o.u[3 * i + 2] = i == 2 ? 1.0f : 0.0f;
+      }
     } else {
       // sigma_i = |F v_i| / |v_i| in FP64: a Rayleigh quotient, second order
       // in the direction error of the FP32 v_i, with the norm of v_i (1 up
@@ -519,10 +534,6 @@ __device__ __forceinline__ void svd3(const T* f, const float* f32, SvdOut<T>& o,
         o.s[i] *= (T)sg;
       }
     }
-    const float top = fmaxf(fmaxf(fabsf(a[0][0]), fabsf(a[1][1])), fabsf(a[2][2]));
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-      o.e[i] = top < 0.25f && o.s[i] > 0.5f ? __fdividef(a[i][i], 1.0f + (float)o.s[i]) : (float)o.s[i] - 1.0f;
   }
 }
 
@@ -563,17 +574,22 @@ __device__ __forceinline__ void quad_weights(float fx, float* w) {
 
 // Fixed-corotated stress from a (U, s, V) decomposition of F, mpm.wgsl:532-599:
 // s_c = clamp(s, 0.1, 10), R = U V^T, J = prod s_c, hardening h by rheology,
-// P = 2 mu h (Fc - R) + lam h (J - 1) cof, S = -dt vol P Fc^T.  With Fc = U Sc
-// V^T and cof = U diag(J/sc) V^T that is S = -dt vol U diag(tau) U^T, tau_i = 2
-// mu h (sc_i - 1) sc_i + lam h (J - 1) J (the Kirchhoff stress in the principal
-// frame): a quarter of the arithmetic, and sc_i - 1 and J - 1, formed in FP64
-// or from the FP32 form's e, keep their relative precision at small strain
-// where Fc - R cancels.  A node at offset d (in metres) receives w (m v + B d)
-// with B = m C + 4/dx^2 S; what is returned is Bd = B dx, the change of that
-// momentum from one node to the next along each axis (the record's form).
-template <class T>
+// P = 2 mu h (Fc - R) + lam h (J - 1) cof, S = -dt vol P Fc^T.  A node at offset
+// d (in metres) receives w (m v + B d) with B = m C + 4/dx^2 S.
+//
+// With Fc = U Sc V^T and cof = U diag(J/sc) V^T, S = -dt vol U diag(tau) U^T, tau_i
+// = 2 mu h (sc_i - 1) sc_i + lam h (J - 1) J (the Kirchhoff stress in the principal
+// frame): a quarter of the arithmetic (FP32 gather at 4M particles 356 -> 300
+// us), and no cancellation in Fc - R.  The FP64 form takes sc_i - 1 and J - 1 in
+// FP64, so that small strains keep their relative precision.
+//
+// FIXED (the fixed-order mode): B, with the stress as the reference writes it,
+// so that runs recorded by any earlier build replay bit for bit; otherwise B dx,
+// the change of a node's momentum from one node to the next along each axis (the
+// record's form).
+template <bool FIXED, class T>
 __device__ __forceinline__ void p2g_affine(const SvdOut<T>& svd, const MatDev& md, float jp, float mass, float vol,
-                                           const float* C, float dt, float dx, float inv_dx, float* Bd) {
+                                           const float* C, float dt, float dx, float inv_dx, float* B) {
   float sc[3], e[3], J, jm1;
   if constexpr (sizeof(T) == 8) {
     double scd[3];
@@ -590,29 +606,59 @@ __device__ __forceinline__ void p2g_affine(const SvdOut<T>& svd, const MatDev& m
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
       sc[i] = clampf(svd.s[i], 0.1f, 10.0f);
-      e[i] = sc[i] == svd.s[i] ? svd.e[i] : sc[i] - 1.0f;
+      e[i] = sc[i] - 1.0f;
     }
-    const float e01 = e[0] + e[1] + e[0] * e[1];
-    jm1 = e01 + e[2] + e01 * e[2];
     J = sc[0] * sc[1] * sc[2];
+    jm1 = J - 1.0f;
   }
   const float h = md.rheo == 2 ? 1.0f : expf(clampf(md.rheo == 1 ? -md.hardening * jp : jp, -3.0f, 3.0f));
-  const float k1 = 2.0f * md.mu * h;
-  const float kv = md.lam * h * jm1 * J;
-  float tau[3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i) tau[i] = k1 * e[i] * sc[i] + kv;
   const float* u = svd.u;
-  const float k = -dt * vol * 4.0f * inv_dx;
-  const float mdx = mass * dx;
+  if constexpr (FIXED && sizeof(T) == 4) {
+    const float* v = svd.v;
+    const float mu_h = md.mu * h;
+    const float lam_h = md.lam * h;
+    const float cofd[3] = {sc[1] * sc[2], sc[0] * sc[2], sc[0] * sc[1]};
+    float Fc[9], cof[9];
+    sandwich(u, sc, v, Fc);
+    sandwich(u, cofd, v, cof);
+    const float k1 = 2.0f * mu_h;
+    const float k2 = lam_h * (J - 1.0f);
+    const float k3 = -dt * vol;
+    float P[9];
 #pragma unroll
-  for (int c = 0; c < 3; ++c)
+    for (int c = 0; c < 3; ++c)
 #pragma unroll
-    for (int r = c; r < 3; ++r) {
-      const float S = k * (u[r] * tau[0] * u[c] + u[3 + r] * tau[1] * u[3 + c] + u[6 + r] * tau[2] * u[6 + c]);
-      Bd[3 * c + r] = mdx * C[3 * c + r] + S;
-      if (r != c) Bd[3 * r + c] = mdx * C[3 * r + c] + S;
-    }
+      for (int r = 0; r < 3; ++r) {
+        // R = U V^T
+        const float Rcr = u[r] * v[c] + u[3 + r] * v[3 + c] + u[6 + r] * v[6 + c];
+        P[3 * c + r] = k3 * (k1 * (Fc[3 * c + r] - Rcr) + k2 * cof[3 * c + r]);
+      }
+    // S = P Fc^T : S[c][r] = sum_k P[k][r] * Fc[k][c]
+    const float four_inv_dx2 = 4.0f * inv_dx * inv_dx;
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        const float S = P[r] * Fc[c] + P[3 + r] * Fc[3 + c] + P[6 + r] * Fc[6 + c];
+        B[3 * c + r] = mass * C[3 * c + r] + four_inv_dx2 * S;
+      }
+  } else {
+    const float k1 = 2.0f * md.mu * h;
+    const float kv = md.lam * h * jm1 * J;
+    float tau[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) tau[i] = k1 * e[i] * sc[i] + kv;
+    const float k = FIXED ? -dt * vol * 4.0f * inv_dx * inv_dx : -dt * vol * 4.0f * inv_dx;
+    const float mc = FIXED ? mass : mass * dx;
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int r = c; r < 3; ++r) {
+        const float S = k * (u[r] * tau[0] * u[c] + u[3 + r] * tau[1] * u[3 + c] + u[6 + r] * tau[2] * u[6 + c]);
+        B[3 * c + r] = mc * C[3 * c + r] + S;
+        if (r != c) B[3 * r + c] = mc * C[3 * r + c] + S;
+      }
+  }
 }
 
 // Plasticity return mapping on (U, s, V), mpm.wgsl:1366-1479.  Writes the
@@ -687,7 +733,6 @@ __device__ __forceinline__ bool plasticity_project(SvdOut<T>& svd, const MatDev&
     if (x != svd.s[a]) {
       changed = true;
       svd.s[a] = x;
-      if constexpr (sizeof(T) == 4) svd.e[a] = x - 1.0f;
     }
   }
   jp = jp_replace ? jp_new : clampf(jp + dq, 0.0f, 5.0f);

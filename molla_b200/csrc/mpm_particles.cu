@@ -27,7 +27,9 @@
 // by the return mapping is reused for the next substep's stress; the first
 // substep of every step_n call runs a record-only gather that computes it
 // from F.
+#include <algorithm>
 #include <cstdint>
+#include <type_traits>
 #include <cuda_runtime.h>
 
 #include "mpm_device.cuh"
@@ -203,6 +205,7 @@ struct GatherCtx {
   int rx, ry, rz;
   uint32_t publish_vc;
   uint32_t start, count;
+  uint32_t tiles;  // sparse storage: the tiles the unit's records touch (block_tiles)
 };
 
 // One particle: G2P + F update + return mapping (MODE != kRecord) and the
@@ -211,8 +214,8 @@ struct GatherCtx {
 // (origin node ctx.rx, ctx.ry, ctx.rz).  Inputs are read when they are needed
 // (mass, volume, J_p and material would hold four registers through the G2P
 // and the SVD); `done` is called after the last of them.
-template <int MODE, bool WRITE_KEYS, class SR, class IN, class DONE>
-__device__ __forceinline__ void particle_step(const PoolDev& p, const SceneDev& sc, uint32_t s, const GatherCtx& ctx,
+template <int MODE, bool WRITE_KEYS, bool SPARSE, bool FIXED, class SR, class IN, class DONE>
+__device__ __forceinline__ void particle_step(const PoolDev& p, const SceneDev& sc, uint32_t s, GatherCtx& ctx,
                                               const float4* __restrict__ vblock, SR stol, int sweeps,
                                               const IN in, DONE&& done, float4 (&rec)[4]) {
   constexpr bool kGather = MODE != kRecord;
@@ -246,10 +249,11 @@ __device__ __forceinline__ void particle_step(const PoolDev& p, const SceneDev& 
       float G[9];
       if (inside) {
         const float4* __restrict__ blk = &vblock[lx0 + 8 * ly0 + 64 * lz0];
-        if constexpr (sizeof(SR) == 4) {
-          // In pairs (one instruction for two sums) in the FP32 form; the FP64
-          // form has no registers left for them (it spilled 164 bytes and the
-          // 16M gather went from 1.19 to 1.36 ms, where the FP32 one gained 6%).
+        if constexpr (sizeof(SR) == 4 && !SPARSE && !FIXED) {
+          // In pairs (one instruction for two sums) in the dense FP32 form; the
+          // others have no registers left for them (the FP64 form spilled 164
+          // bytes and the 16M gather went from 1.19 to 1.36 ms, where the FP32
+          // one gained 6%).
           // The sums over k, then j, then i of the products with the weights
           // (and, for one axis at a time, with the offset d), the components in
           // pairs: (x, y) of sum w gv, z of it beside z of sum w d_z gv, (x, y)
@@ -408,22 +412,23 @@ __device__ __forceinline__ void particle_step(const PoolDev& p, const SceneDev& 
           bool changed = true;
           const SR s_trial[3] = {svd.s[0], svd.s[1], svd.s[2]};
           if (plasticity_project<SR>(svd, md, jp_new, changed)) {
-            // The trial F stays when the return mapping left every singular
-            // value unchanged; otherwise U diag(s - s_trial) V^T is added to
-            // it: the reference's F = U s V^T in exact arithmetic (F = U
-            // s_trial V^T), with the FP32 rounding of U and V scaled by the
-            // (small) change in s instead of by F.  Finite: s lies in [0.05,
-            // 20] and F = U s_trial V^T.
-            if (changed) {
+            // The FP32 form rebuilds F = U s V^T every substep (the reference).
+            // The FP64 form keeps the trial F when the return mapping left
+            // every singular value unchanged, and otherwise adds U diag(s -
+            // s_trial) V^T to it: the same F in exact arithmetic (F = U s_trial
+            // V^T), with the FP32 rounding of U and V scaled by the (small)
+            // change in s instead of by F.  Finite: s lies in [0.05, 20] and F
+            // = U s_trial V^T.
+            if (changed || sizeof(SR) == 4) {
               float ds[3];
 #pragma unroll
-              for (int i = 0; i < 3; ++i) ds[i] = (float)(svd.s[i] - s_trial[i]);
+              for (int i = 0; i < 3; ++i) ds[i] = sizeof(SR) == 4 ? (float)svd.s[i] : (float)(svd.s[i] - s_trial[i]);
 #pragma unroll
               for (int c = 0; c < 3; ++c)
 #pragma unroll
                 for (int r = 0; r < 3; ++r)
-                  F[3 * c + r] += (svd.u[r] * ds[0]) * svd.v[c] + (svd.u[3 + r] * ds[1]) * svd.v[3 + c] +
-                                  (svd.u[6 + r] * ds[2]) * svd.v[6 + c];
+                  F[3 * c + r] = (sizeof(SR) == 4 ? 0.0f : F[3 * c + r]) + (svd.u[r] * ds[0]) * svd.v[c] +
+                                 (svd.u[3 + r] * ds[1]) * svd.v[3 + c] + (svd.u[6 + r] * ds[2]) * svd.v[6 + c];
             }
             jp = jp_new;
           } else {
@@ -495,6 +500,7 @@ __device__ __forceinline__ void particle_step(const PoolDev& p, const SceneDev& 
       // (the reference's m v + B d with d = ((i, j, k) - fx) dx regrouped:
       // node (i, j, k) receives w (m, q + i Bdx + j Bdy + k Bdz)).  A particle
       // that faulted deposits nothing: mass 0, at a position off every grid.
+      // FIXED: the fixed-order mode's own form (p2g_affine).
       float Bd[9];
 #pragma unroll
       for (int i = 0; i < 9; ++i) Bd[i] = 0.f;
@@ -505,23 +511,38 @@ __device__ __forceinline__ void particle_step(const PoolDev& p, const SceneDev& 
           for (int i = 0; i < 9; ++i) Fs[i] = (SR)F[i];
           svd3<SR>(Fs, F, svd, stol, sweeps);
         }
-        p2g_affine<SR>(svd, sc.mat[mat], jp, mass, vol, C, sc.dt, sc.dx, sc.inv_dx, Bd);
+        p2g_affine<FIXED, SR>(svd, sc.mat[mat], jp, mass, vol, C, sc.dt, sc.dx, sc.inv_dx, Bd);
       }
       const float mr = ok ? mass : 0.f;
-      float q[3];
+      if constexpr (FIXED) {
+        rec[0] = make_float4(x, y, z, mr);
+        rec[1] = make_float4(ok ? mass * v[0] : 0.f, ok ? mass * v[1] : 0.f, ok ? mass * v[2] : 0.f, Bd[0]);
+        rec[2] = make_float4(Bd[1], Bd[2], Bd[3], Bd[4]);
+        rec[3] = make_float4(Bd[5], Bd[6], Bd[7], Bd[8]);
+      } else {
+        float q[3];
 #pragma unroll
-      for (int r = 0; r < 3; ++r) {
-        q[r] = ok ? mass * v[r] : 0.f;
+        for (int r = 0; r < 3; ++r) {
+          q[r] = ok ? mass * v[r] : 0.f;
 #pragma unroll
-        for (int a = 0; a < 3; ++a) q[r] -= (ok ? xq[a] - bf[a] : 0.f) * Bd[3 * a + r];
+          for (int a = 0; a < 3; ++a) q[r] -= (ok ? xq[a] - bf[a] : 0.f) * Bd[3 * a + r];
       }
-      rec[0] = make_float4(mr, q[0], q[1], q[2]);
-      rec[1] = make_float4(Bd[0], Bd[1], Bd[2], Bd[3]);
-      rec[2] = make_float4(Bd[4], Bd[5], Bd[6], Bd[7]);
-      rec[3] = make_float4(Bd[8], mr != 0.f ? xq[0] : kOffGrid, xq[1], xq[2]);
+        rec[0] = make_float4(mr, q[0], q[1], q[2]);
+        rec[1] = make_float4(Bd[0], Bd[1], Bd[2], Bd[3]);
+        rec[2] = make_float4(Bd[4], Bd[5], Bd[6], Bd[7]);
+        rec[3] = make_float4(Bd[8], mr != 0.f ? xq[0] : kOffGrid, xq[1], xq[2]);
+      }
       // sparse storage: the tiles this record's deposit will touch
-      if (sc.tile_cap && ok)
-        mark_stencil_tiles(sc, p.tile_mark, (int)bf[0] - sc.winx, (int)bf[1] - sc.winy, (int)bf[2] - sc.winz);
+      if (SPARSE && sc.tile_cap && ok) {
+        const int bx = (int)bf[0] - sc.winx, by = (int)bf[1] - sc.winy, bz = (int)bf[2] - sc.winz;
+        const int lx = bx - ctx.rx, ly = by - ctx.ry, lz = bz - ctx.rz;
+        if ((unsigned)lx <= 5u && (unsigned)ly <= 5u && (unsigned)lz <= 5u) {
+          const uint32_t bits = block_tiles(lx, ly, lz);
+          if (bits & ~ctx.tiles) atomicOr(&ctx.tiles, bits);
+        } else {
+          mark_far_tiles(sc, p.tile_mark, bx, by, bz);
+        }
+      }
     }
     if constexpr (WRITE_KEYS) {
       const int win[3] = {sc.winx, sc.winy, sc.winz};
@@ -535,12 +556,13 @@ __device__ __forceinline__ void particle_step(const PoolDev& p, const SceneDev& 
 
 // A gather warp's shared memory: the velocity block, the particle inputs of
 // its lanes' next round ([input][lane], the staged order), the scene record.
-template <bool GATHER>
+template <bool GATHER, bool SPARSE>
 struct __align__(128) GatherWarp {
   float4 vel[GATHER ? kRegionNodes : 1];
   float in[kStagedInputs][32];
   SceneDev sc;
   GatherCtx ctx;
+  uint32_t slots[SPARSE ? 27 : 1];  // sparse storage: slots of the tiles around the unit's, or kNoSlot
   uint32_t scene;   // scene whose record sc holds
   uint32_t parity;  // of the velocity block's next arrival
   uint64_t bar;
@@ -561,17 +583,20 @@ struct __align__(128) GatherWarp {
 // and the dependent chains of the SVD; a quarter of the DRAM rate.  Against a
 // CTA per tile with a barrier per item: 1.26 -> 1.19 ms at 16M particles (FP64
 // SVD, 256^3), 333 -> 278 us at 4M and 63 -> 52 us at 500k (FP32).
-template <int MODE, bool WRITE_KEYS, class SR>
+// SPARSE: the group holds scenes on sparse storage (the tile lookups and marks
+// cost the dense form up to 20% in registers and code: 278 -> 340 us at 4M).
+template <int MODE, bool WRITE_KEYS, bool SPARSE, bool FIXED, class SR>
 __global__ void __launch_bounds__(kGatherThreads, 5) k_g2p(PoolDev p, double tol, int sweeps,
                                                             int publish_all) {
   constexpr bool kGather = MODE != kRecord;
   constexpr bool kScatter = MODE != kG2P;
   constexpr uint32_t kWarps = kGatherThreads / 32;
-  __shared__ GatherWarp<kGather> s_warp[kWarps];
+  __shared__ GatherWarp<kGather, SPARSE> s_warp[kWarps];
   const uint32_t lane = threadIdx.x & 31u;
-  GatherWarp<kGather>& w = s_warp[threadIdx.x >> 5];
+  GatherWarp<kGather, SPARSE>& w = s_warp[threadIdx.x >> 5];
   if (lane == 0) {
     w.scene = 0xffffffffu;
+    w.ctx.tiles = 0;
     w.parity = 0;
     mbar_init(&w.bar, 1);
     fence_mbar_init();
@@ -627,10 +652,10 @@ __global__ void __launch_bounds__(kGatherThreads, 5) k_g2p(PoolDev p, double tol
       const uint32_t tx = unit.tile % tw, ty = (unit.tile / tw) % tw, tz = unit.tile / (tw * tw);
       const int rx = 4 * (int)tx - 1, ry = 4 * (int)ty - 1, rz = 4 * (int)tz - 1;
       if (lane == 0)
-        w.ctx = GatherCtx{status, rx, ry, rz, (publish_all || budget_ends(status)) ? 1u : 0u, unit.start, unit.count};
+        w.ctx = GatherCtx{status, rx, ry, rz, (publish_all || budget_ends(status)) ? 1u : 0u, unit.start, unit.count, 0u};
       if constexpr (kGather) {
         // Stage the 8^3-node velocity block (out-of-grid nodes read as zero).
-        if (sc.tile_cap == 0 && sc.n >= (uint32_t)kRegion) {
+        if ((!SPARSE || sc.tile_cap == 0) && sc.n >= (uint32_t)kRegion) {
           if (lane == 0) {
             fence_proxy_async_smem();  // the lanes' reads of the block are done (__syncwarp below)
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(&w.bar)),
@@ -649,7 +674,31 @@ __global__ void __launch_bounds__(kGatherThreads, 5) k_g2p(PoolDev p, double tol
           }
           __syncwarp();
           if (lane == 0) w.parity = parity ^ 1u;
+        } else if (SPARSE && sc.tile_cap) {
+          // the slots of the 27 tiles around, then every node by cp.async
+          if (lane < 27u) {
+            const int ax = (int)tx + (int)(lane % 3u) - 1, ay = (int)ty + (int)((lane / 3u) % 3u) - 1,
+                      az = (int)tz + (int)(lane / 9u) - 1;
+            const bool in = (unsigned)ax < tw && (unsigned)ay < tw && (unsigned)az < tw;
+            w.slots[lane] =
+                in ? p.tile_slot[sc.key_off + (uint32_t)ax + tw * ((uint32_t)ay + tw * (uint32_t)az)] : kNoSlot;
+          }
+          __syncwarp();
+#pragma unroll 4
+          for (uint32_t r = lane; r < (uint32_t)kRegionNodes; r += 32) {
+            // region coordinate l is node 4t - 1 + l: tile (l + 3) / 4 - 1, node (l + 3) % 4 in it
+            const uint32_t lx = (r & 7u) + 3u, ly = ((r >> 3) & 7u) + 3u, lz = (r >> 6) + 3u;
+            const uint32_t slot = w.slots[(lx >> 2) + 3u * (ly >> 2) + 9u * (lz >> 2)];
+            const bool in = slot != kNoSlot && (unsigned)(rx + (int)lx - 3) < sc.n &&
+                            (unsigned)(ry + (int)ly - 3) < sc.n && (unsigned)(rz + (int)lz - 3) < sc.n;
+            if (in)
+              cp_async16(&w.vel[r], p.vel + sc.grid_off + 64ull * slot + (lx & 3u) + 4u * (ly & 3u) + 16u * (lz & 3u));
+            else
+              w.vel[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+          }
+          cp_async_wait_all();
         } else {
+          // a grid of fewer than 8 nodes an axis
           for (uint32_t r = lane; r < (uint32_t)kRegionNodes; r += 32) {
             const int64_t c =
                 node_index(sc, p.tile_slot, rx + (int)(r & 7u), ry + (int)((r >> 3) & 7u), rz + (int)(r >> 6));
@@ -662,7 +711,7 @@ __global__ void __launch_bounds__(kGatherThreads, 5) k_g2p(PoolDev p, double tol
         cp_async_wait_all();
         const uint32_t s = w.ctx.start + k;
         float4 rec[4];
-        particle_step<MODE, WRITE_KEYS, SR>(
+        particle_step<MODE, WRITE_KEYS, SPARSE, FIXED, SR>(
             p, sc, s, w.ctx, w.vel, stol, sweeps, StagedIn{&w.in[0][lane]},
             [&] { fetch(k + 32u, w.ctx.start, w.ctx.count); }, rec);
         if constexpr (kScatter) {
@@ -676,6 +725,20 @@ __global__ void __launch_bounds__(kGatherThreads, 5) k_g2p(PoolDev p, double tol
     }
     cp_async_wait_all();
     __syncwarp();
+    if constexpr (kScatter && SPARSE) {
+      // sparse storage: one store per tile the unit touched
+      if (sc.tile_cap) {
+        const uint32_t tw = sc.w;
+        const uint32_t ax = (uint32_t)((w.ctx.rx + 1) >> 2) + lane % 3u - 1u,
+                       ay = (uint32_t)((w.ctx.ry + 1) >> 2) + (lane / 3u) % 3u - 1u,
+                       az = (uint32_t)((w.ctx.rz + 1) >> 2) + lane / 9u - 1u;
+        if (lane < 27u && (w.ctx.tiles >> lane & 1u) && ax < tw && ay < tw && az < tw)
+          p.tile_mark[sc.key_off + ax + tw * (ay + tw * az)] = 1;
+        __syncwarp();
+        if (lane == 0) w.ctx.tiles = 0;  // a frozen scene's unit marks none
+      }
+      __syncwarp();
+    }
     u = __shfl_sync(0xffffffffu, next, 0);
   }
 }
@@ -1106,7 +1169,7 @@ __global__ void __launch_bounds__(kFusedThreads, 2) k_g2p2g(PoolDev p, double to
         atomicOr(s_item.status, kFaultDeviceWait);
       }
       s_ctx = GatherCtx{s_item.status, s_item.rx, s_item.ry, s_item.rz, budget_ends(s_item.status) ? 1u : 0u,
-                        item.start, item.count};
+                        item.start, item.count, 0u};
     }
     __syncthreads();
     // Stage the 8^3-node velocity block (out-of-grid nodes read as zero).
@@ -1122,7 +1185,7 @@ __global__ void __launch_bounds__(kFusedThreads, 2) k_g2p2g(PoolDev p, double to
       for (uint32_t k = threadIdx.x; k < item.count; k += kFusedThreads) {
         const uint32_t s = item.start + k;
         float4 rec[4];
-        particle_step<kG2PRecord, WRITE_KEYS, SR>(p, s_sc, s, s_ctx, s_vel, stol, sweeps, PoolIn{p, s}, [] {},
+        particle_step<kG2PRecord, WRITE_KEYS, false, false, SR>(p, s_sc, s, s_ctx, s_vel, stol, sweeps, PoolIn{p, s}, [] {},
                                                   rec);
         stage_store(s_stage, k, rec);
       }
@@ -1152,6 +1215,8 @@ __global__ void __launch_bounds__(kScatterThreads, 2) k_p2g_det(PoolDev p, float
   __shared__ uint32_t s_first[64], s_end[64];
   __shared__ float s_part[3 * 64 * 9 * 4];
   __shared__ uint32_t s_fault;
+  launch_next();
+  wait_previous();
   const float4* __restrict__ rec = reinterpret_cast<const float4*>(p.rec);
   const uint32_t n32 = p.n_items[0];
   const uint32_t n_items = n32 + p.n_items[1];
@@ -1162,6 +1227,7 @@ __global__ void __launch_bounds__(kScatterThreads, 2) k_p2g_det(PoolDev p, float
     const Item item = p.items[slot];
     const SceneDev* __restrict__ scp = p.scenes + item.scene;
     const uint32_t w = scp->w;
+    const float ox = scp->ox, oy = scp->oy, oz = scp->oz, inv_dx = scp->inv_dx, dx = scp->dx;
     const int winx = scp->winx, winy = scp->winy, winz = scp->winz;
     uint32_t* status = p.status + (size_t)scp->status * kStatusWords;
     const uint32_t tx = item.tile % w, ty = (item.tile / w) % w, tz = item.tile / (w * w);
@@ -1185,40 +1251,52 @@ __global__ void __launch_bounds__(kScatterThreads, 2) k_p2g_det(PoolDev p, float
       const int cx = cell & 3, cy = (cell >> 2) & 3, cz = cell >> 4;
       const int bx = 4 * (int)tx + cx, by = 4 * (int)ty + cy, bz = 4 * (int)tz + cz;  // this cell's base
       const int win[3] = {winx, winy, winz};
-      for (uint32_t s = s_first[cell]; s < s_end[cell]; ++s) {
-        const float4 c0 = __ldg(&rec[4 * (size_t)s]);
-        if (c0.x == 0.f) continue;
-        const float4 c1 = __ldg(&rec[4 * (size_t)s + 1]);
-        const float4 c2 = __ldg(&rec[4 * (size_t)s + 2]);
-        const float4 c3 = __ldg(&rec[4 * (size_t)s + 3]);
-        const float mass = c0.x;
-        const float xp[3] = {c3.y, c3.z, c3.w};
-        float wgt[3][3];
+      const uint32_t end = s_end[cell];
+      uint32_t s = s_first[cell];
+      float4 n0, n1, n2, n3;  // the next record, loaded while this one is added
+      auto load = [&](uint32_t at) {
+        const float4* r = rec + 4 * (size_t)at;
+        n0 = __ldg(r);
+        n1 = __ldg(r + 1);
+        n2 = __ldg(r + 2);
+        n3 = __ldg(r + 3);
+      };
+      if (s < end) load(s);
+      for (; s < end; ++s) {
+        const float4 r0 = n0, r1 = n1, r2 = n2, r3 = n3;
+        if (s + 1 < end) load(s + 1);
+        if (r0.w == 0.f) continue;
+        const float mass = r0.w;
+        const float B[9] = {r1.w, r2.x, r2.y, r2.z, r2.w, r3.x, r3.y, r3.z, r3.w};
+        const float xp[3] = {lattice_pos(r0.x, ox, inv_dx), lattice_pos(r0.y, oy, inv_dx),
+                             lattice_pos(r0.z, oz, inv_dx)};
+        float wgt[3][3], fx[3];
         int base[3];
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
           const float bf = floorf(xp[a] - 0.5f);
           base[a] = (int)bf - win[a];
-          quad_weights(xp[a] - bf, wgt[a]);
+          fx[a] = xp[a] - bf;
+          quad_weights(fx[a], wgt[a]);
         }
         const float wi = slab == 0 ? wgt[0][0] : (slab == 1 ? wgt[0][1] : wgt[0][2]);
-        const float fs = (float)slab;
-        const float qx[3] = {c0.y + fs * c1.x, c0.z + fs * c1.y, c0.w + fs * c1.z};
+        const float di = ((float)slab - fx[0]) * dx;
+        const float qx[3] = {r1.x + B[0] * di, r1.y + B[1] * di, r1.z + B[2] * di};
         const bool own = base[0] == bx && base[1] == by && base[2] == bz;
         if (!own && slab == 0 && threadIdx.x < 64) atomicOr(status, kFaultNondeterministic);
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
           const float wij = wi * wgt[1][j];
-          const float fj = (float)j;
-          const float qy[3] = {qx[0] + fj * c1.w, qx[1] + fj * c2.x, qx[2] + fj * c2.y};
+          const float dj = ((float)j - fx[1]) * dx;
+          const float qy[3] = {qx[0] + B[3] * dj, qx[1] + B[4] * dj, qx[2] + B[5] * dj};
 #pragma unroll
           for (int kk = 0; kk < 3; ++kk) {
             const float wt = wij * wgt[2][kk];
-            const float fk = (float)kk;
+            const float dk = ((float)kk - fx[2]) * dx;
             const float dm = wt * mass;
-            const float px = wt * (qy[0] + fk * c2.z);
-            const float py = wt * (qy[1] + fk * c2.w);
-            const float pz = wt * (qy[2] + fk * c3.x);
+            const float px = wt * (qy[0] + B[6] * dk);
+            const float py = wt * (qy[1] + B[7] * dk);
+            const float pz = wt * (qy[2] + B[8] * dk);
             if (own) {
               am[3 * j + kk] += dm;
               apx[3 * j + kk] += px;
@@ -1277,59 +1355,62 @@ __global__ void __launch_bounds__(kScatterThreads, 2) k_p2g_det(PoolDev p, float
 // it, summed in (tz, ty, tx) order by the first such tile's thread.
 __global__ void k_combine_det(PoolDev p, const float4* __restrict__ blocks, const uint32_t* __restrict__ tile_item,
                               int acc_out) {
-  const uint32_t n32 = p.n_items[0];
-  if (blockIdx.x >= n32 + p.n_items[1]) return;
-  const uint32_t it = item_slot(p, n32, blockIdx.x);  // the item's slot, as tile_item holds it
-  const Item item = p.items[it];
-  const SceneDev* __restrict__ scp = p.scenes + item.scene;
-  const int w = (int)scp->w, n = (int)scp->n;
-  const uint32_t key_off = scp->key_off;
-  const int tx = (int)(item.tile % (uint32_t)w), ty = (int)((item.tile / (uint32_t)w) % (uint32_t)w),
-            tz = (int)(item.tile / (uint32_t)(w * w));
-  for (int q = threadIdx.x; q < kTileNodes; q += blockDim.x) {
-    const int g[3] = {4 * tx + q % 6, 4 * ty + (q / 6) % 6, 4 * tz + q / 36};
-    if (g[0] >= n || g[1] >= n || g[2] >= n) continue;
-    int lo[3], hi[3];
+  launch_next();
+  wait_previous();
+  const uint32_t n32 = p.n_items[0], total = n32 + p.n_items[1];
+  for (uint32_t li = blockIdx.x; li < total; li += gridDim.x) {
+    const uint32_t it = item_slot(p, n32, li);  // the item's slot, as tile_item holds it
+    const Item item = p.items[it];
+    const SceneDev* __restrict__ scp = p.scenes + item.scene;
+    const int w = (int)scp->w, n = (int)scp->n;
+    const uint32_t key_off = scp->key_off;
+    const int tx = (int)(item.tile % (uint32_t)w), ty = (int)((item.tile / (uint32_t)w) % (uint32_t)w),
+              tz = (int)(item.tile / (uint32_t)(w * w));
+    for (int q = threadIdx.x; q < kTileNodes; q += blockDim.x) {
+      const int g[3] = {4 * tx + q % 6, 4 * ty + (q / 6) % 6, 4 * tz + q / 36};
+      if (g[0] >= n || g[1] >= n || g[2] >= n) continue;
+      int lo[3], hi[3];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      hi[a] = g[a] / 4;
-      lo[a] = max(0, (g[a] - 5 + 3) / 4);  // smallest t with 4t + 5 >= g
-      hi[a] = min(hi[a], w - 1);
-    }
-    bool mine = false, found = false;
-    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int cz = lo[2]; cz <= hi[2]; ++cz)
-      for (int cy = lo[1]; cy <= hi[1]; ++cy)
-        for (int cx = lo[0]; cx <= hi[0]; ++cx) {
-          const uint32_t key = key_off + (uint32_t)(cx + w * (cy + w * cz));
-          const uint32_t other = tile_item[key];
-          if (other == 0xffffffffu) continue;
-          if (!found) {
-            found = true;
-            mine = other == it;
-            if (!mine) break;
+      for (int a = 0; a < 3; ++a) {
+        hi[a] = g[a] / 4;
+        lo[a] = max(0, (g[a] - 5 + 3) / 4);  // smallest t with 4t + 5 >= g
+        hi[a] = min(hi[a], w - 1);
+      }
+      bool mine = false, found = false;
+      float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int cz = lo[2]; cz <= hi[2]; ++cz)
+        for (int cy = lo[1]; cy <= hi[1]; ++cy)
+          for (int cx = lo[0]; cx <= hi[0]; ++cx) {
+            const uint32_t key = key_off + (uint32_t)(cx + w * (cy + w * cz));
+            const uint32_t other = tile_item[key];
+            if (other == 0xffffffffu) continue;
+            if (!found) {
+              found = true;
+              mine = other == it;
+              if (!mine) break;
+            }
+            const int l = (g[0] - 4 * cx) + 6 * ((g[1] - 4 * cy) + 6 * (g[2] - 4 * cz));
+            const float4 b = blocks[(size_t)other * kTileNodes + l];
+            sum.x += b.x;
+            sum.y += b.y;
+            sum.z += b.z;
+            sum.w += b.w;
           }
-          const int l = (g[0] - 4 * cx) + 6 * ((g[1] - 4 * cy) + 6 * (g[2] - 4 * cz));
-          const float4 b = blocks[(size_t)other * kTileNodes + l];
-          sum.x += b.x;
-          sum.y += b.y;
-          sum.z += b.z;
-          sum.w += b.w;
-        }
-    const int64_t c = mine ? node_index(*scp, p.tile_slot, g[0], g[1], g[2]) : -1;
-    if (c >= 0) {
-      // One writer per node; the cell holds zero or out-of-order deposits.
-      float4& a = p.acc[acc_out][c];
-      const float4 old = a;
-      a = make_float4(old.x + sum.x, old.y + sum.y, old.z + sum.z, old.w + sum.w);
-      touch(p.touched[acc_out], (uint64_t)c);
+      const int64_t c = mine ? node_index(*scp, p.tile_slot, g[0], g[1], g[2]) : -1;
+      if (c >= 0) {
+        // One writer per node; the cell holds zero or out-of-order deposits.
+        float4& a = p.acc[acc_out][c];
+        const float4 old = a;
+        a = make_float4(old.x + sum.x, old.y + sum.y, old.z + sum.z, old.w + sum.w);
+        touch(p.touched[acc_out], (uint64_t)c);
+      }
     }
   }
 }
 
 // ---------------------------------------------------------------------------
 
-template <int MODE, bool KEYS, class SR>
+template <int MODE, bool KEYS, bool SPARSE, bool FIXED, class SR>
 static cudaError_t launch_gather_t(const PoolDev& p, double tol, int sweeps, int grid, cudaStream_t st,
                                    bool publish_all) {
   if (MODE == kRecord) {
@@ -1337,25 +1418,32 @@ static cudaError_t launch_gather_t(const PoolDev& p, double tol, int sweeps, int
     const cudaError_t e = cudaMemsetAsync(p.work, 0, kWorkWords * sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
   }
-  return launch_dependent(k_g2p<MODE, KEYS, SR>, grid, kGatherThreads, 0, st, p, tol, sweeps, publish_all ? 1 : 0);
+  return launch_dependent(k_g2p<MODE, KEYS, SPARSE, FIXED, SR>, grid, kGatherThreads, 0, st, p, tol, sweeps,
+                          publish_all ? 1 : 0);
 }
 
-cudaError_t launch_gather(int mode, bool write_keys, bool svd_fp64, const PoolDev& p, double tol, int sweeps,
-                          int grid, cudaStream_t st, bool publish_all) {
-#define MPM_DISPATCH(M)                                                                          \
-  if (mode == M) {                                                                               \
-    if (svd_fp64) {                                                                              \
-      return write_keys ? launch_gather_t<M, true, double>(p, tol, sweeps, grid, st, publish_all) \
-                        : launch_gather_t<M, false, double>(p, tol, sweeps, grid, st, publish_all); \
-    }                                                                                            \
-    return write_keys ? launch_gather_t<M, true, float>(p, tol, sweeps, grid, st, publish_all) \
-                      : launch_gather_t<M, false, float>(p, tol, sweeps, grid, st, publish_all); \
+cudaError_t launch_gather(int mode, bool write_keys, bool sparse, bool fixed, bool svd_fp64, const PoolDev& p,
+                          double tol, int sweeps, int grid, cudaStream_t st, bool publish_all) {
+  auto pick = [&](auto m) {
+    constexpr int M = decltype(m)::value;
+    auto with = [&](auto keys, auto sp, auto fx) {
+      constexpr bool K = decltype(keys)::value, S = decltype(sp)::value, X = decltype(fx)::value;
+      return svd_fp64 ? launch_gather_t<M, K, S, X, double>(p, tol, sweeps, grid, st, publish_all)
+                      : launch_gather_t<M, K, S, X, float>(p, tol, sweeps, grid, st, publish_all);
+    };
+    const std::true_type yes;
+    const std::false_type no;
+    // the fixed-order mode takes the sparse form, which serves dense scenes too
+    if (fixed) return write_keys ? with(yes, yes, yes) : with(no, yes, yes);
+    if (write_keys) return sparse ? with(yes, yes, no) : with(yes, no, no);
+    return sparse ? with(no, yes, no) : with(no, no, no);
+  };
+  switch (mode) {
+    case kRecord: return pick(std::integral_constant<int, kRecord>{});
+    case kG2P: return pick(std::integral_constant<int, kG2P>{});
+    case kG2PRecord: return pick(std::integral_constant<int, kG2PRecord>{});
+    default: return cudaErrorInvalidValue;
   }
-  MPM_DISPATCH(kRecord)
-  MPM_DISPATCH(kG2P)
-  MPM_DISPATCH(kG2PRecord)
-#undef MPM_DISPATCH
-  return cudaErrorInvalidValue;
 }
 
 constexpr size_t kFusedStageBytes = (size_t)kStageMax * 64;
@@ -1455,15 +1543,14 @@ cudaError_t launch_scatter(const PoolDev& p, const CUtensorMap& rec_map, int acc
 }
 
 cudaError_t launch_scatter_det(const PoolDev& p, float4* blocks, int acc_out, int grid, cudaStream_t st) {
-  k_p2g_det<<<grid, kScatterThreads, 0, st>>>(p, blocks, acc_out);
-  return cudaGetLastError();
+  return launch_dependent(k_p2g_det, grid, kScatterThreads, 0, st, p, blocks, acc_out);
 }
 
 cudaError_t launch_combine_det(const PoolDev& p, const float4* blocks, const uint32_t* tile_item, uint32_t max_items,
                                int acc_out, cudaStream_t st) {
   if (!max_items) return cudaSuccess;
-  k_combine_det<<<max_items, 128, 0, st>>>(p, blocks, tile_item, acc_out);
-  return cudaGetLastError();
+  return launch_dependent(k_combine_det, (int)std::min<uint32_t>(max_items, 148u * 16u), 128, 0, st, p, blocks, tile_item,
+                          acc_out);
 }
 
 static int persistent(const void* fn, int threads, size_t dyn_smem = 0) {
@@ -1477,8 +1564,8 @@ static int persistent(const void* fn, int threads, size_t dyn_smem = 0) {
 }
 
 int gather_grid_size(bool svd_fp64) {
-  return svd_fp64 ? persistent((const void*)k_g2p<kG2PRecord, false, double>, kGatherThreads)
-                  : persistent((const void*)k_g2p<kG2PRecord, false, float>, kGatherThreads);
+  return svd_fp64 ? persistent((const void*)k_g2p<kG2PRecord, false, false, false, double>, kGatherThreads)
+                  : persistent((const void*)k_g2p<kG2PRecord, false, false, false, float>, kGatherThreads);
 }
 
 int fused_grid_size(bool svd_fp64) {

@@ -827,7 +827,7 @@ void Group::launch_gather_pass(int mode, bool keys, cudaStream_t st, bool publis
   eng->prof_begin(mode == kRecord ? kStageRecord : kStageGather, st, &pr);
   for (int f64 = 0; f64 < 2; ++f64) {
     if (!(f64 ? any_svd64() : any_svd32())) continue;
-    MPM_CK(launch_gather(mode, keys, f64 != 0, pool(), f64 ? svd_tol64 : svd_tol32, svd_sweeps,
+    MPM_CK(launch_gather(mode, keys, any_sparse(), deterministic, f64 != 0, pool(), f64 ? svd_tol64 : svd_tol32, svd_sweeps,
                          gather_grid(f64 != 0), st, publish_all));
     eng->launches += 1;
   }
