@@ -750,7 +750,7 @@ __global__ void __launch_bounds__(kGatherThreads, 5) k_g2p(PoolDev p, double tol
 // record mass is zero (numerical fault this substep) deposit nothing.
 //
 // Persistent CTAs over items (a tile's particles from the last regrouping,
-// at most kStageMax), 192 threads.  Per item:
+// at most kStageMax), 224 threads.  Per item:
 //  1. stage: the item's 64-byte records (contiguous slots) arrive in shared
 //     memory as 2-D TMA tiles of 64 records (cp.async.bulk.tensor completing
 //     on an mbarrier), issued while the previous item's block was flushed.
@@ -1105,7 +1105,7 @@ __global__ void __launch_bounds__(kScatterThreads, 4) k_p2g(PoolDev p, const __g
     // for the counter or the descriptor.
     uint32_t next = 0;
     if (threadIdx.x == 0) next = gridDim.x + atomicAdd(p.work + kWorkScatter, 1u);
-    const uint32_t share = core_share(p.item_order + (size_t)f.slot * 64);
+    const uint32_t share = threadIdx.x < 192 ? core_share(p.item_order + (size_t)f.slot * 64) : 0u;
     const bool staged = f.count - 1u < (uint32_t)kStageMax;
     const bool ok = staged && mbar_wait_bounded(&s_bar, parity);
     const bool live = ok && f.live != 0u;
@@ -1229,7 +1229,7 @@ __global__ void __launch_bounds__(kFusedThreads, 2) k_g2p2g(PoolDev p, double to
 // The result depends only on the scene's own particles and identities: it is
 // bit-identical from run to run and whether or not other scenes share the
 // launch.
-__global__ void __launch_bounds__(kScatterThreads, 2) k_p2g_det(PoolDev p, float4* __restrict__ blocks, int acc_out) {
+__global__ void __launch_bounds__(kDetThreads, 2) k_p2g_det(PoolDev p, float4* __restrict__ blocks, int acc_out) {
   __shared__ uint32_t s_first[64], s_end[64];
   __shared__ float s_part[3 * 64 * 9 * 4];
   __shared__ uint32_t s_fault;
@@ -1561,7 +1561,7 @@ cudaError_t launch_scatter(const PoolDev& p, const CUtensorMap& rec_map, int acc
 }
 
 cudaError_t launch_scatter_det(const PoolDev& p, float4* blocks, int acc_out, int grid, cudaStream_t st) {
-  return launch_dependent(k_p2g_det, grid, kScatterThreads, 0, st, p, blocks, acc_out);
+  return launch_dependent(k_p2g_det, grid, kDetThreads, 0, st, p, blocks, acc_out);
 }
 
 cudaError_t launch_combine_det(const PoolDev& p, const float4* blocks, const uint32_t* tile_item, uint32_t max_items,
