@@ -157,6 +157,11 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(smem)), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
 
 // Waits for the phase of `bar` with the given parity to complete; gives up
 // (returns false) after about one second.
@@ -191,6 +196,14 @@ struct PoolIn {
   __device__ __forceinline__ uint32_t mat() const { return p.meta[s] & 7u; }
 };
 constexpr int kInMass = 12, kInVol = 13, kInJp = 14;
+// What particle_step tells the owner of its inputs: `late` before it reads the
+// first of mass, volume, J_p and material, `early_read` when it has read x and F
+// for the last time, `done` when it has read everything.
+struct NoRefill {
+  __device__ __forceinline__ void late() const {}
+  __device__ __forceinline__ void early_read() const {}
+  __device__ __forceinline__ void done() const {}
+};
 // Lattice x of a record that deposits nothing: outside every grid.
 constexpr float kOffGrid = 1.0e30f;
 static_assert(PY == PX + 1 && PZ == PX + 2 && MASS == F0 + 9 && VOL == F0 + 10 && JP == F0 + 11,
@@ -213,11 +226,11 @@ struct GatherCtx {
 // uniform values; vblock is the staged 8^3-node velocity block of its tile
 // (origin node ctx.rx, ctx.ry, ctx.rz).  Inputs are read when they are needed
 // (mass, volume, J_p and material would hold four registers through the G2P
-// and the SVD); `done` is called after the last of them.
-template <int MODE, bool WRITE_KEYS, bool SPARSE, bool FIXED, class SR, class IN, class DONE>
+// and the SVD).
+template <int MODE, bool WRITE_KEYS, bool SPARSE, bool FIXED, class SR, class IN, class REFILL>
 __device__ __forceinline__ void particle_step(const PoolDev& p, const SceneDev& sc, uint32_t s, GatherCtx& ctx,
                                               const float4* __restrict__ vblock, SR stol, int sweeps,
-                                              const IN in, DONE&& done, float4 (&rec)[4]) {
+                                              const IN in, const REFILL refill, float4 (&rec)[4]) {
   constexpr bool kGather = MODE != kRecord;
   constexpr bool kScatter = MODE != kG2P;
   float x, y, z, F[9], jp;
@@ -361,6 +374,7 @@ __device__ __forceinline__ void particle_step(const PoolDev& p, const SceneDev& 
       v[0] = vs[0];
       v[1] = vs[1];
       v[2] = vs[2];
+      refill.late();
       const MatDev& md = sc.mat[in.mat()];
       if (md.rheo == 2) {
         v[0] *= md.vfac;
@@ -374,6 +388,7 @@ __device__ __forceinline__ void particle_step(const PoolDev& p, const SceneDev& 
       z = in.f(2);
 #pragma unroll
       for (int i = 0; i < 9; ++i) F[i] = in.f(3 + i);
+      refill.early_read();
       float np[3] = {x + sc.dt * v[0], y + sc.dt * v[1], z + sc.dt * v[2]};
       // F <- (I + dt C) F
       float A[9];
@@ -469,6 +484,8 @@ __device__ __forceinline__ void particle_step(const PoolDev& p, const SceneDev& 
     z = in.f(2);
 #pragma unroll
     for (int i = 0; i < 9; ++i) F[i] = in.f(3 + i);
+    refill.late();
+    refill.early_read();
     v[0] = plane(p, VX)[s];
     v[1] = plane(p, VY)[s];
     v[2] = plane(p, VZ)[s];
@@ -487,7 +504,7 @@ __device__ __forceinline__ void particle_step(const PoolDev& p, const SceneDev& 
   }
   const uint32_t mat = in.mat();
   const float mass = in.f(kInMass), vol = in.f(kInVol);
-  done();
+  refill.done();
   if constexpr (kScatter || WRITE_KEYS) {
     // lattice coordinates of the new position
     const float xq[3] = {lattice_pos(x, sc.ox, sc.inv_dx), lattice_pos(y, sc.oy, sc.inv_dx),
@@ -615,23 +632,35 @@ __global__ void __launch_bounds__(kGatherThreads, 5) k_g2p(PoolDev p, double tol
     uint32_t next = 0;  // this warp's next unit, taken now and read after this one's work
     if (lane == 0) next = lo + kWarps * gridDim.x + atomicAdd(p.work + (sizeof(SR) == 8 ? kWorkGather64 : kWorkGather32), 1u);
     // The inputs of a lane's next particle are copied to shared memory
-    // (cp.async) from the moment this one's are consumed; those of its first
+    // (cp.async) from the moment this one's are consumed -- x and F before the
+    // SVD, the rest before the stress -- and waited for apart: x and F as a
+    // round begins, the rest after its G2P.  Those of a lane's first particle
     // are requested here, so that their loads overlap the velocity block's.
-    auto fetch = [&](uint32_t k, uint32_t start, uint32_t count) {
+    auto fetch_early = [&](uint32_t k, uint32_t start, uint32_t count) {
       if (k < count) {
-        const uint32_t s = start + k;
-        // walk the planes with one pointer: PX..PZ, then F0..JP
+        // walk the planes with one pointer: PX..PZ, then F0..F8
         const size_t cap = p.cap;
-        const float* src = p.planes + s;
+        const float* src = p.planes + (start + k);
 #pragma unroll
         for (int q = 0; q < 3; ++q, src += cap) cp_async4(&w.in[q][lane], src);
         src += (size_t)(F0 - 3) * cap;
 #pragma unroll
-        for (int q = 3; q < kStagedInputs - 1; ++q, src += cap) cp_async4(&w.in[q][lane], src);
-        cp_async4(&w.in[kStagedInputs - 1][lane], p.meta + s);
+        for (int q = 3; q < kInMass; ++q, src += cap) cp_async4(&w.in[q][lane], src);
       }
+      cp_async_commit();
     };
-    fetch(lane, unit.start, unit.count);
+    auto fetch_late = [&](uint32_t k, uint32_t start, uint32_t count) {
+      if (k < count) {
+        const size_t cap = p.cap;
+        const float* src = p.planes + (size_t)MASS * cap + (start + k);
+#pragma unroll
+        for (int q = kInMass; q < kStagedInputs - 1; ++q, src += cap) cp_async4(&w.in[q][lane], src);
+        cp_async4(&w.in[kStagedInputs - 1][lane], p.meta + (start + k));
+      }
+      cp_async_commit();
+    };
+    fetch_early(lane, unit.start, unit.count);
+    fetch_late(lane, unit.start, unit.count);
     if (unit.scene != w.scene) {
       const uint32_t* src = reinterpret_cast<const uint32_t*>(p.scenes + unit.scene);
       uint32_t* dst = reinterpret_cast<uint32_t*>(&w.sc);
@@ -708,12 +737,21 @@ __global__ void __launch_bounds__(kGatherThreads, 5) k_g2p(PoolDev p, double tol
       }
       __syncwarp();
       for (uint32_t k = lane; k < w.ctx.count; k += 32) {
-        cp_async_wait_all();
+        cp_async_wait<1>();
         const uint32_t s = w.ctx.start + k;
+        auto early = [&] { fetch_early(k + 32u, w.ctx.start, w.ctx.count); };
+        auto rest = [&] { fetch_late(k + 32u, w.ctx.start, w.ctx.count); };
+        struct Refill {
+          decltype(early)& e;
+          decltype(rest)& l;
+          __device__ __forceinline__ void late() const { cp_async_wait<0>(); }
+          __device__ __forceinline__ void early_read() const { e(); }
+          __device__ __forceinline__ void done() const { l(); }
+        };
         float4 rec[4];
         particle_step<MODE, WRITE_KEYS, SPARSE, FIXED, SR>(
-            p, sc, s, w.ctx, w.vel, stol, sweeps, StagedIn{&w.in[0][lane]},
-            [&] { fetch(k + 32u, w.ctx.start, w.ctx.count); }, rec);
+            p, sc, s, w.ctx, w.vel, stol, sweeps, StagedIn{&w.in[0][lane]}, Refill{early, rest},
+            rec);
         if constexpr (kScatter) {
           float4* r4 = reinterpret_cast<float4*>(p.rec) + 4 * (size_t)s;
           r4[0] = rec[0];
@@ -948,16 +986,15 @@ __device__ __forceinline__ void add_node(ScatterShared& ss, int r, float2 xy, fl
 // (k_item_order), which deals the cells so that a warp's 30 flush atomics of
 // one node and channel fall on 30 different shared-memory banks, in
 // particle-count order inside the warp (scatter -18% against a plain count
-// order).  Then all T threads share the (margin cell, slab) pairs of the
-// non-empty cells particles moved into.  A thread adds the nine slab nodes of
+// order).  The (margin cell, slab) pairs of the non-empty cells particles moved
+// into go to the warps beyond the core's from the start, then to all.  A thread adds the nine slab nodes of
 // its cell's particles in registers and issues 9 x 4 shared-memory atomics for
 // the whole cell; no two lanes of a warp add to the same node.
 template <int T>
 __device__ __forceinline__ void deposit_item(const float4* stage, uint32_t share, const ScatterItem& f,
                                              ScatterShared& ss) {
   static_assert(T >= 192, "the core cells take 6 warps of 10 cells x 3 slabs");
-  // One loop (one copy of the code) over the core pairs, then the (margin
-  // cell, slab) pairs of the non-empty margin cells.
+  // One loop (one copy of the code) over the core pairs, then the margin's.
 #pragma unroll 1
   for (uint32_t u = threadIdx.x; u < 192u + 3u * ss.n_margin; u += T) {
     if (u >= 192u) share = ss.margin[(u - 192u) / 3u] + (((u - 192u) % 3u) << 8);
@@ -1203,7 +1240,7 @@ __global__ void __launch_bounds__(kFusedThreads, 2) k_g2p2g(PoolDev p, double to
       for (uint32_t k = threadIdx.x; k < item.count; k += kFusedThreads) {
         const uint32_t s = item.start + k;
         float4 rec[4];
-        particle_step<kG2PRecord, WRITE_KEYS, false, false, SR>(p, s_sc, s, s_ctx, s_vel, stol, sweeps, PoolIn{p, s}, [] {},
+        particle_step<kG2PRecord, WRITE_KEYS, false, false, SR>(p, s_sc, s, s_ctx, s_vel, stol, sweeps, PoolIn{p, s}, NoRefill{},
                                                   rec);
         stage_store(s_stage, k, rec);
       }
