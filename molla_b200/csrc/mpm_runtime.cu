@@ -302,6 +302,7 @@ void Group::invalidate_graphs() {
   for (auto& kv : graphs)
     if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
   graphs.clear();
+  graph_seen.clear();
   ++epoch;
 }
 
@@ -745,6 +746,12 @@ static int bits_for(uint64_t values) {
   while (b < 32 && ((1ull << b) - 1ull) <= values) ++b;
   return b;
 }
+// bits of the values 0 .. top
+static int bits_up_to(uint64_t top) {
+  int b = 1;
+  while (b < 32 && (top >> b) != 0) ++b;
+  return b;
+}
 
 // Regrouping: sort (base-cell key, identity) stably — key = (scene tile
 // offset + 4^3 tile of the base cell, cell inside the tile) — and move the
@@ -761,10 +768,15 @@ void Group::regroup(bool compute_keys, cudaStream_t st, bool move_records) {
     eng->launches += 1;
   }
   const uint32_t n_sort = (uint32_t)ids.high_water();
+  // Removed particles' all-ones keys need a pattern of their own above every
+  // live key; without any, the live keys' bits do (2^24 of them on a 256^3
+  // grid: three passes, not four).
+  const uint64_t key_values = (uint64_t)key_space << kCellBits;
+  const bool none_removed = n_sort == n_live && n_retiring == 0;
   uint32_t* skeys = nullptr;
   uint32_t* sids = nullptr;
   MPM_CK(radix_sort_pairs(st, keys_by_id.ptr, nullptr, ks[0].ptr, ks[1].ptr, vs[0].ptr, vs[1].ptr, hist.ptr, n_sort,
-                          bits_for((uint64_t)key_space << kCellBits), &skeys, &sids, &eng->launches));
+                          none_removed ? bits_up_to(key_values ? key_values - 1 : 0) : bits_for(key_values), &skeys, &sids, &eng->launches));
   // both record buffers exist only in deterministic mode (set_deterministic)
   if (move_records && (rec[0].count < (size_t)16 * cap || rec[1].count < (size_t)16 * cap))
     throw Error(MPM_ERR_INVALID, "MPM regroup: records can move only between two allocated record buffers");
@@ -1207,6 +1219,21 @@ void Group::step_graph(uint32_t substeps, uint32_t repeat, cudaStream_t st, cuda
     auto it = graphs.find(key);
     Graph g;
     if (it == graphs.end() || it->second.epoch != epoch) {
+      // A sequence is captured the second time it is asked for in a layout:
+      // capturing and instantiating one costs several times its launches (20
+      // substeps: about 2 ms against 0.3), and a served tick after an
+      // admission or a retirement is often never seen again.
+      cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+      MPM_CK(cudaStreamIsCapturing(st, &capture));
+      uint64_t& seen = graph_seen[key];
+      if (seen != epoch && capture == cudaStreamCaptureStatusNone) {
+        seen = epoch;
+        if (ev_begin && r == 0) MPM_CK(cudaEventRecord(ev_begin, st));
+        run_substeps(substeps, st);
+        if (ev_end && r + 1 == repeat) MPM_CK(cudaEventRecord(ev_end, st));
+        finish_retirements();
+        continue;
+      }
       const auto t_build0 = std::chrono::steady_clock::now();
       const uint64_t saved = eng->launches;
       cudaGraph_t graph = nullptr;
