@@ -155,7 +155,9 @@ __global__ void __launch_bounds__(kCellThreads, 4) k_grid_update(PoolDev p, cons
   wait_previous();
   if (blockIdx.x == 0 && threadIdx.x < (unsigned)kWorkWords) p.work[threadIdx.x] = 0u;
   if (threadIdx.x < 32) {
-    const uint64_t blk = (uint64_t)blockIdx.x * per_cta + threadIdx.x;
+    // every gridDim-th pool block: those with work lie together (a box of
+    // particles, the first slots of sparse storage)
+    const uint64_t blk = (uint64_t)threadIdx.x * gridDim.x + blockIdx.x;
     const bool exists = (int)threadIdx.x < per_cta && blk * kCellThreads < total_cells;
     Work wk{(uint32_t)blk, exists ? block_scene[blk] : 0xffffffffu, 0u, 0u};
     const bool in_a = exists && p.touched[acc_in][blk] != 0;
@@ -290,19 +292,27 @@ __global__ void __launch_bounds__(kCellThreads) k_grid_jacobi(PoolDev p, const u
   const uint32_t local = (uint32_t)local64;
   const uint32_t q = local / n;
   const int ix = (int)(local - q * n), iy = (int)(q % n), iz = (int)(q / n);
+  // The six neighbours' masses and velocities are all requested before the
+  // first is tested (one round trip instead of up to twelve: a sweep is latency).
   const int off[6][3] = {{1, 0, 0}, {-1, 0, 0}, {0, 1, 0}, {0, -1, 0}, {0, 0, 1}, {0, 0, -1}};
-  float ax = 0.f, ay = 0.f, az = 0.f, count = 0.f;
+  float nm[6];
+  float4 nv[6];
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
     const int nx = ix + off[k][0], ny = iy + off[k][1], nz = iz + off[k][2];
-    if ((unsigned)nx >= n || (unsigned)ny >= n || (unsigned)nz >= n) continue;
-    const uint64_t ng = sc.grid_off + (uint64_t)nx + (uint64_t)n * ((uint64_t)ny + (uint64_t)n * (uint64_t)nz);
-    const float nm = p.acc[acc_in][ng].x;
-    if (nm <= 1.0e-9f || !(nm == nm)) continue;
-    const float4 nv = src[ng];
-    ax = ax + nv.x;
-    ay = ay + nv.y;
-    az = az + nv.z;
+    const bool in = (unsigned)nx < n && (unsigned)ny < n && (unsigned)nz < n;
+    const uint64_t ng =
+        in ? sc.grid_off + (uint64_t)nx + (uint64_t)n * ((uint64_t)ny + (uint64_t)n * (uint64_t)nz) : g;
+    nm[k] = in ? p.acc[acc_in][ng].x : 0.f;
+    nv[k] = src[ng];
+  }
+  float ax = 0.f, ay = 0.f, az = 0.f, count = 0.f;
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    if (nm[k] <= 1.0e-9f || !(nm[k] == nm[k])) continue;
+    ax = ax + nv[k].x;
+    ay = ay + nv[k].y;
+    az = az + nv[k].z;
     count = count + 1.0f;
   }
   if (count > 0.f) {
