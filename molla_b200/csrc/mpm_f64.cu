@@ -22,7 +22,7 @@
 // is a serial chain of square roots), latency of the list walk in k64_p2g.  With
 // a thread per particle issuing 108 global atomics, its own SVD there, and
 // separate g2p and plasticity kernels a substep of 132,651 particles on a 64^3
-// grid took 165 us of kernels; it takes 72.
+// grid took 165 us of kernels; it takes 69.
 #include <algorithm>
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -328,8 +328,10 @@ __global__ void __launch_bounds__(256) k64_grid(Scene64 sc, State64 st, int par,
 // GATHER: g2p, plasticity and the record for the next p2g (into the lists of
 // parity `par`; a call's last substep makes none); otherwise the record of the
 // state as it is.
+// Four blocks an SM (128 registers, 116 bytes spilled) beat three at 168: 43 -> 37
+// us for 132,651 particles, which are 2.3 waves of the latter.
 template <bool GATHER>
-__global__ void __launch_bounds__(128) k64_particle(Scene64 sc, State64 st, int par, int last) {
+__global__ void __launch_bounds__(128, 4) k64_particle(Scene64 sc, State64 st, int par, int last) {
   launch_next();
   wait_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
