@@ -57,7 +57,8 @@ constexpr int kGridTogether = 4;
 // has 1,024 in all), up to 32 where most blocks are idle and reading their
 // marks a few bytes per thread block is what costs (a 256^3 grid with 13% of
 // its blocks touched: 90 -> 56 us; sparse storage of 65,536 tiles, 1,450 of them
-// active: 37 us -> under 10).
+// active: 37 -> 6, taken in a stride, since those with work lie together; 23 with
+// 32 consecutive blocks a thread block).
 constexpr int kGridMaxPerCta = 32;
 inline int grid_blocks_per_cta(uint64_t pool_blocks) {
   const uint64_t want = pool_blocks / (148 * 4) / kGridTogether * kGridTogether;
