@@ -262,11 +262,11 @@ __device__ __forceinline__ void particle_step(const PoolDev& p, const SceneDev& 
       float G[9];
       if (inside) {
         const float4* __restrict__ blk = &vblock[lx0 + 8 * ly0 + 64 * lz0];
-        if constexpr (sizeof(SR) == 4 && !SPARSE && !FIXED) {
-          // In pairs (one instruction for two sums) in the dense FP32 form; the
-          // others have no registers left for them (the FP64 form spilled 164
-          // bytes and the 16M gather went from 1.19 to 1.36 ms, where the FP32
-          // one gained 6%).
+        if constexpr ((sizeof(SR) == 4 || !SPARSE) && !FIXED) {
+          // In pairs, one instruction for two sums (16M particles x 16 substeps
+          // 38.2 -> 37.6 ms in the FP64 form, 4M x 12 6.63 -> 6.43 in the FP32
+          // form); the sparse FP64 form has no registers left for them (184
+          // bytes of spills).
           // The sums over k, then j, then i of the products with the weights
           // (and, for one axis at a time, with the offset d), the components in
           // pairs: (x, y) of sum w gv, z of it beside z of sum w d_z gv, (x, y)
