@@ -10,8 +10,9 @@
 //     zero, so skipping them leaves the permutation unchanged);
 //   * each pass is three kernels: a per-tile digit histogram with
 //     warp-aggregated shared-memory counts, a per-digit scan of the tile
-//     counts (one CTA per digit), and a scatter that ranks keys stably
-//     inside the tile with __match_any_sync and a per-warp prefix;
+//     counts (one CTA per digit; few tiles do without, kSelfScan), and a
+//     scatter that ranks keys stably inside the tile with __match_any_sync
+//     and a per-warp prefix;
 //   * pass 0 can generate the identity values (0..n-1) itself.
 #include <algorithm>
 #include <cstdint>
@@ -42,10 +43,16 @@ constexpr int kRounds = kSortTile / kThreads;  // 16
 constexpr int kSmallRounds = 4;
 constexpr uint32_t kSmallTile = kSmallRounds * kThreads;
 constexpr uint32_t kSmallSort = 1u << 20;
+// Up to this many tiles a scatter block adds up the histograms itself (one
+// coalesced read of them, 32 tiles in flight), which drops the scan's launch and
+// its round trip; beyond, that reading grows with the square of the tiles.
+// 98 tiles (100k particles regrouped every substep, 3 passes each, 32 substeps):
+// 7.93 -> 7.60 ms; 130 tiles: even.
+constexpr uint32_t kSelfScan = 160;
 
 template <int ROUNDS>
 __global__ void __launch_bounds__(kThreads) k_sort_hist(const uint32_t* __restrict__ keys, uint32_t n, int shift,
-                                                   uint32_t nblocks, uint32_t* __restrict__ hist) {
+                                                   uint32_t nblocks, uint32_t* __restrict__ hist, int by_tile) {
   __shared__ uint32_t s_h[kBins + 1];
   launch_next();
   wait_previous();
@@ -63,7 +70,8 @@ __global__ void __launch_bounds__(kThreads) k_sort_hist(const uint32_t* __restri
     if (lane == __ffs(peers) - 1 && d < (uint32_t)kBins) atomicAdd(&s_h[d], (uint32_t)__popc(peers));
   }
   __syncthreads();
-  hist[(size_t)tid * nblocks + blockIdx.x] = s_h[tid];
+  // [digit][tile] for the scan, [tile][digit] for blocks that add it up themselves
+  hist[by_tile ? (size_t)blockIdx.x * kBins + tid : (size_t)tid * nblocks + blockIdx.x] = s_h[tid];
 }
 
 // One CTA per digit: exclusive scan of hist[d][0..nblocks) in place, total to
@@ -116,7 +124,7 @@ __global__ void __launch_bounds__(kThreads) k_sort_scatter(const uint32_t* __res
                                                       uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
                                                       uint32_t n, int shift, uint32_t nblocks,
                                                       const uint32_t* __restrict__ hist,
-                                                      const uint32_t* __restrict__ totals) {
+                                                      const uint32_t* __restrict__ totals, int by_tile) {
   __shared__ uint32_t s_base[kBins];           // global base of each digit for this tile
   __shared__ uint32_t s_cnt[kWarps][kBins];    // per-warp digit counts of the current round
   __shared__ uint32_t s_pre[kWarps][kBins];    // per-warp digit prefix of the current round
@@ -128,7 +136,18 @@ __global__ void __launch_bounds__(kThreads) k_sort_scatter(const uint32_t* __res
 
   // Exclusive scan of the digit totals (256 values) -> digit base.
   {
-    const uint32_t x = totals[tid];
+    uint32_t x = 0, before = 0;  // the digit's keys in all tiles, and in those before this one
+    if (by_tile) {
+#pragma unroll 32
+      for (uint32_t b = 0; b < nblocks; ++b) {
+        const uint32_t h = hist[(size_t)b * kBins + tid];
+        x += h;
+        before += b < blockIdx.x ? h : 0u;
+      }
+    } else {
+      x = totals[tid];
+      before = hist[(size_t)tid * nblocks + blockIdx.x];
+    }
     uint32_t inc = x;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -139,7 +158,7 @@ __global__ void __launch_bounds__(kThreads) k_sort_scatter(const uint32_t* __res
     __syncthreads();
     uint32_t off = 0;
     for (int w = 0; w < warp; ++w) off += s_wsum[w];
-    s_base[tid] = off + inc - x + hist[(size_t)tid * nblocks + blockIdx.x];
+    s_base[tid] = off + inc - x + before;
   }
   for (int w = 0; w < kWarps; ++w) s_cnt[w][tid] = 0;
   __syncthreads();
@@ -219,15 +238,15 @@ cudaError_t radix_sort_pairs(cudaStream_t stream, const uint32_t* keys_in, const
     const int shift = 8 * p;
     kout = (p % 2 == 0) ? keys_a : keys_b;
     vout = (p % 2 == 0) ? vals_a : vals_b;
-    const int nb = (int)nblocks;
+    const int nb = (int)nblocks, by_tile = small && nblocks <= kSelfScan ? 1 : 0;
     cudaError_t e = launch_dependent(small ? k_sort_hist<kSmallRounds> : k_sort_hist<kRounds>, nb, kThreads, 0, stream, kin,
-                                     n, shift, nblocks, hist);
-    if (e == cudaSuccess) e = launch_dependent(k_sort_scan, kBins, 1024, 0, stream, hist, nblocks, totals);
+                                     n, shift, nblocks, hist, by_tile);
+    if (e == cudaSuccess && !by_tile) e = launch_dependent(k_sort_scan, kBins, 1024, 0, stream, hist, nblocks, totals);
     if (e == cudaSuccess)
       e = launch_dependent(small ? k_sort_scatter<kSmallRounds> : k_sort_scatter<kRounds>, nb, kThreads, 0, stream, kin, vin,
-                           iota, kout, vout, n, shift, nblocks, hist, totals);
+                           iota, kout, vout, n, shift, nblocks, hist, totals, by_tile);
     if (e != cudaSuccess) return e;
-    if (launches) *launches += 3;
+    if (launches) *launches += by_tile ? 2 : 3;
     kin = kout;
     vin = vout;
     iota = 0;
@@ -366,9 +385,9 @@ extern "C" int mpm_radix_sort_pairs_noalloc(uint32_t* d_keys, uint32_t* d_values
     const uint32_t* vin = to_scratch ? d_values : svals;
     uint32_t* kout = to_scratch ? skeys : d_keys;
     uint32_t* vout = to_scratch ? svals : d_values;
-    k_sort_hist<kRounds><<<nblocks, kThreads, 0, st>>>(kin, n, 8 * p, nblocks, hist);
+    k_sort_hist<kRounds><<<nblocks, kThreads, 0, st>>>(kin, n, 8 * p, nblocks, hist, 0);
     k_sort_scan<<<kBins, 1024, 0, st>>>(hist, nblocks, totals);
-    k_sort_scatter<kRounds><<<nblocks, kThreads, 0, st>>>(kin, vin, 0, kout, vout, n, 8 * p, nblocks, hist, totals);
+    k_sort_scatter<kRounds><<<nblocks, kThreads, 0, st>>>(kin, vin, 0, kout, vout, n, 8 * p, nblocks, hist, totals, 0);
   }
   if (passes % 2 == 1) {
     cudaMemcpyAsync(d_keys, skeys, (size_t)n * 4, cudaMemcpyDeviceToDevice, st);
