@@ -6,27 +6,27 @@
 //
 //   grid_update(n)  acc[a] -> velocity, clears acc[b]               (grid sweep)
 //   gather(n)       G2P(n) + F update + return mapping(n); writes the particle
-//                   and, for the next substep, the APIC/stress matrix
-//                   B = m C + 4/dx^2 S (S the fixed-corotated stress term)
+//                   and, for the next substep, its 64-byte record in deposit
+//                   form (mass, m v - fx.Bd, Bd = B dx with the APIC/stress
+//                   matrix B = m C + 4/dx^2 S, S the fixed-corotated stress)
 //   scatter(n+1)    27-node deposit of mass and momentum into acc[b]
 //
-// Both particle kernels are persistent over a work list of (scene, tile, slot
-// range) items built by the last regrouping (a stable radix sort of the
-// particles by base-cell key; tiles of 4^3 base cells, cut into items of at
-// most kStageMax particles).  The gather stages the 8^3-node velocity block
-// around the tile in shared memory; the scatter stages the item's 64-byte
-// records with one bulk copy, bins them by their current base cell and
-// accumulates into an 8^3-node shared block that it flushes to HBM with one
-// float4 atomic per non-empty node.  For large groups they are separate
-// kernels because the gather (SVD, return mapping) needs ~128 registers per
-// thread while the scatter needs fewer: split, each runs at its own
-// occupancy, and the B record's round trip through HBM is cheaper than the
-// fused kernel's lower occupancy.  For small groups (a few hundred items,
-// about one wave) the fused k_g2p2g keeps the records in shared memory and
-// saves a launch per substep.  The SVD computed
-// by the return mapping is reused for the next substep's stress; the first
-// substep of every step_n call runs a record-only gather that computes it
-// from F.
+// Both particle kernels are persistent over lists built by the last
+// regrouping (a stable radix sort of the particles by base-cell key, in tiles
+// of 4^3 base cells).  The gather's warps each take units (32..640 particles
+// of a tile) with the tile's 8^3-node velocity block in shared memory; the
+// scatter's CTAs take items (at most kStageMax particles of a tile), stage the
+// records with TMA, link them into lists by their current base cell and
+// accumulate into an 8^3-node shared block that is flushed to HBM with one
+// float4 atomic per non-empty node.  They are separate kernels because the
+// gather (SVD, return mapping) runs at 96 registers in warps that wait for
+// nobody, while the scatter's steps need CTA barriers: split, each has its own
+// shape, and the record's round trip through HBM is cheaper than the fused
+// kernel's two CTAs an SM.  Up to kFusedMaxParticles the fused k_g2p2g keeps
+// the records in shared memory and saves a launch per substep.  The SVD
+// computed by the return mapping is reused for the next substep's stress; a
+// step_n call whose records cannot be carried over from the last one opens
+// with a record-only gather that computes it from F.
 #include <algorithm>
 #include <cstdint>
 #include <type_traits>
@@ -594,12 +594,13 @@ struct __align__(128) GatherWarp {
 // the list, its first by its index and each later one from the counter, with
 // the velocity block of the unit's tile fetched into its own shared memory by
 // one TMA box, and shares no barrier with the other warps of its CTA.
-// What bounds it: instruction issue (60% of the slots; 64 warp instructions a
-// particle of mixed materials) and, behind that, instruction fetch -- the
-// kernel was 55 KB, of which a second SVD for a case that never came was 13 --
-// and the dependent chains of the SVD; a quarter of the DRAM rate.  Against a
-// CTA per tile with a barrier per item: 1.26 -> 1.19 ms at 16M particles (FP64
-// SVD, 256^3), 333 -> 278 us at 4M and 63 -> 52 us at 500k (FP32).
+// What bounds it: instruction issue (64% of the slots; 61 warp instructions a
+// particle of mixed materials) and, behind that, the dependent chains of the
+// SVD and instruction fetch (41 KB of code; it was 55, of which a second SVD
+// for a case that never came was 13); 0.4 of the DRAM rate.  From a CTA per
+// tile with a barrier per item, over all changes: 1.26 -> 1.13 ms at 16M
+// particles (FP64 SVD, 256^3), 333 -> 279 us at 4M and 63 -> 52 us at 500k
+// (FP32), with the records in deposit form.
 // SPARSE: the group holds scenes on sparse storage (the tile lookups and marks
 // cost the dense form up to 20% in registers and code: 278 -> 340 us at 4M).
 template <int MODE, bool WRITE_KEYS, bool SPARSE, bool FIXED, class SR>
@@ -805,8 +806,9 @@ __global__ void __launch_bounds__(kGatherThreads, 5) k_g2p(PoolDev p, double tol
 //     warp), the three slabs of a cell in adjacent lanes, then the non-empty
 //     margin cells particles moved into (listed by step 2).  It
 //     adds the nine slab-i node contributions of its cell's particles in
-//     registers and issues 9 x 4 shared-memory atomics for the whole cell,
-//     not per particle; no two lanes of a warp add to the same node;
+//     registers and adds 9 x 4 sums to the shared block (add_node) for the
+//     whole cell, not per particle; no two lanes of a warp add to the same
+//     node in one step;
 //  4. flush: every non-empty node of the 8^3 block goes to HBM with one
 //     float4 atomic and is cleared for the next item.
 // Every wait on the stage is bounded (about one second); a wait that gives
@@ -817,8 +819,9 @@ __global__ void __launch_bounds__(kGatherThreads, 5) k_g2p(PoolDev p, double tol
 // (15% of DRAM rate).  Lists instead of a counting sort, records written in
 // deposit form by the gather instead of rewritten here, and the item's frame
 // in shared memory took it from 0.832 to 0.773 ms on a 16M-particle scene
-// (256^3), from 0.239 to 0.222 ms at 4M and from 43.3 to 40 us at 500k; the
-// gather pays 0.03 of its 1.26 ms for the form at 16M.
+// (256^3), from 0.239 to 0.222 ms at 4M and from 43.3 to 40 us at 500k (the
+// gather pays 0.03 ms for the form at 16M); swaps in flight together and a
+// warp for the margin cells, to 0.715 and 0.204 ms.
 __device__ __noinline__ void deposit_global(float4 c0, float4 c1, float4 c2, float4 c3, float4* __restrict__ acc,
                                             uint8_t* __restrict__ touched, const SceneDev* __restrict__ scp,
                                             const uint32_t* __restrict__ tile_slot) {
@@ -988,8 +991,8 @@ __device__ __forceinline__ void add_node(ScatterShared& ss, int r, float2 xy, fl
 // particle-count order inside the warp (scatter -18% against a plain count
 // order).  The (margin cell, slab) pairs of the non-empty cells particles moved
 // into go to the warps beyond the core's from the start, then to all.  A thread adds the nine slab nodes of
-// its cell's particles in registers and issues 9 x 4 shared-memory atomics for
-// the whole cell; no two lanes of a warp add to the same node.
+// its cell's particles in registers and adds 9 x 4 sums to the shared block for
+// the whole cell; no two lanes of a warp add to the same node in one step.
 template <int T>
 __device__ __forceinline__ void deposit_item(const float4* stage, uint32_t share, const ScatterItem& f,
                                              ScatterShared& ss) {
