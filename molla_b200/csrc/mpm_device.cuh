@@ -168,6 +168,9 @@ enum Work : int { kWorkGather32 = 0, kWorkGather64 = 1, kWorkScatter = 2, kWorkW
 // the one before them still runs (launch_next allows it as soon as every CTA
 // of the running kernel has started) and wait here for its results before
 // they touch anything it writes.
+// A kernel that waits takes its inputs without __restrict__: a load
+// through a const __restrict__ parameter counts as a read of memory that never
+// changes while the kernel runs, and may be moved above the wait.
 __device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -141,7 +141,7 @@ __device__ __forceinline__ void grid_node(const PoolDev& p, uint32_t sid, const 
   p.vel[g] = make_float4(v[0], v[1], v[2], m);
 }
 
-__global__ void __launch_bounds__(kCellThreads, 4) k_grid_update(PoolDev p, const uint32_t* __restrict__ block_scene,
+__global__ void __launch_bounds__(kCellThreads, 4) k_grid_update(PoolDev p, const uint32_t* block_scene,
                                                               uint64_t total_cells, int per_cta, int acc_in,
                                                               int count_substep) {
   static_assert(kCellThreads == kCellBlock, "one thread per cell of a grid-pool block");
@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(kCellThreads, 4) k_grid_update(PoolDev p, cons
 // sand mass within radius + dx of a sphere adds the reaction
 // -(m w / dt) (v_sphere - v_node) (w tapered linearly over the outer cell)
 // and its torque to the sphere's wrench.
-__global__ void __launch_bounds__(kCellThreads) k_rigid_shell(PoolDev p, const uint32_t* __restrict__ block_scene,
+__global__ void __launch_bounds__(kCellThreads) k_rigid_shell(PoolDev p, const uint32_t* block_scene,
                                                               uint64_t total_cells, int acc_in) {
   launch_next();
   wait_previous();
@@ -268,9 +268,9 @@ __global__ void __launch_bounds__(kCellThreads) k_rigid_shell(PoolDev p, const u
 // face neighbours that carry mass, v = (m v + a v_avg) / (m + a), with
 // a = dt^2 m c^2 / dx^2 and c^2 = E / 1500 (the reference's wave-speed
 // stiffness estimate); massless nodes and scenes whose sweeps are done copy.
-__global__ void __launch_bounds__(kCellThreads) k_grid_jacobi(PoolDev p, const uint32_t* __restrict__ block_scene,
+__global__ void __launch_bounds__(kCellThreads) k_grid_jacobi(PoolDev p, const uint32_t* block_scene,
                                                               uint64_t total_cells, int acc_in,
-                                                              const float4* __restrict__ src, float4* __restrict__ dst,
+                                                              const float4* src, float4* __restrict__ dst,
                                                               uint32_t sweep) {
   launch_next();
   wait_previous();
@@ -412,11 +412,11 @@ __global__ void k_scene_keys(PoolDev p, uint32_t sid, const uint32_t* __restrict
 
 // Physically regroup particles into sorted order: slot s of the new pool
 // receives identity ids[s].
-__global__ void k_reorder(const float* __restrict__ src, float* __restrict__ dst, uint32_t cap,
-                          const uint32_t* __restrict__ meta_src, uint32_t* __restrict__ meta_dst,
+__global__ void k_reorder(const float* src, float* __restrict__ dst, uint32_t cap,
+                          const uint32_t* meta_src, uint32_t* __restrict__ meta_dst,
                           uint32_t* __restrict__ orig_dst, uint32_t* __restrict__ slot_of,
-                          const uint32_t* __restrict__ ids, const uint32_t* __restrict__ keys,
-                          uint32_t* __restrict__ slot_key, const float4* __restrict__ rec_src,
+                          const uint32_t* ids, const uint32_t* keys,
+                          uint32_t* __restrict__ slot_key, const float4* rec_src,
                           float4* __restrict__ rec_dst, uint32_t n_live) {
   launch_next();
   wait_previous();
@@ -568,9 +568,9 @@ __device__ __forceinline__ void item_order_one(const Item* __restrict__ items, u
 // Grid-stride over the work list's items (the FP32-SVD items, then the
 // FP64-SVD ones at the top of the slot range), so that only the items that
 // exist are visited.
-__global__ void __launch_bounds__(64) k_item_order(const Item* __restrict__ items,
-                                                   const uint32_t* __restrict__ n_items, uint32_t item_top,
-                                                   const uint32_t* __restrict__ slot_key,
+__global__ void __launch_bounds__(64) k_item_order(const Item* items,
+                                                   const uint32_t* n_items, uint32_t item_top,
+                                                   const uint32_t* slot_key,
                                                    uint8_t* __restrict__ item_order) {
   __shared__ uint32_t s_cnt[64];
   __shared__ uint8_t s_pair[32][2];
@@ -752,7 +752,7 @@ __global__ void k_tiles_reset(PoolDev p, uint32_t n_scenes) {
 // marks are cleared.  More active tiles than the capacity latch
 // kFaultTileOverflow; the excess tiles get no slot (their deposits are
 // dropped and the scene freezes from the next substep).
-__global__ void k_tiles_finalize(PoolDev p, const uint32_t* __restrict__ key_scene, uint32_t K) {
+__global__ void k_tiles_finalize(PoolDev p, const uint32_t* key_scene, uint32_t K) {
   launch_next();
   wait_previous();
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;

@@ -1275,7 +1275,7 @@ __global__ void __launch_bounds__(kDetThreads, 2) k_p2g_det(PoolDev p, float4* _
   __shared__ uint32_t s_fault;
   launch_next();
   wait_previous();
-  const float4* __restrict__ rec = reinterpret_cast<const float4*>(p.rec);
+  const float4* rec = reinterpret_cast<const float4*>(p.rec);
   const uint32_t n32 = p.n_items[0];
   const uint32_t n_items = n32 + p.n_items[1];
   const int cell = threadIdx.x & 63;
@@ -1411,7 +1411,7 @@ __global__ void __launch_bounds__(kDetThreads, 2) k_p2g_det(PoolDev p, float4* _
 // Combine pass of the deterministic scatter: node g of a scene receives the
 // blocks of the (up to 8) occupied tiles whose footprint [4t, 4t+5] contains
 // it, summed in (tz, ty, tx) order by the first such tile's thread.
-__global__ void k_combine_det(PoolDev p, const float4* __restrict__ blocks, const uint32_t* __restrict__ tile_item,
+__global__ void k_combine_det(PoolDev p, const float4* blocks, const uint32_t* tile_item,
                               int acc_out) {
   launch_next();
   wait_previous();

@@ -51,7 +51,7 @@ constexpr uint32_t kSmallSort = 1u << 20;
 constexpr uint32_t kSelfScan = 160;
 
 template <int ROUNDS>
-__global__ void __launch_bounds__(kThreads) k_sort_hist(const uint32_t* __restrict__ keys, uint32_t n, int shift,
+__global__ void __launch_bounds__(kThreads) k_sort_hist(const uint32_t* keys, uint32_t n, int shift,
                                                    uint32_t nblocks, uint32_t* __restrict__ hist, int by_tile) {
   __shared__ uint32_t s_h[kBins + 1];
   launch_next();
@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(kThreads) k_sort_hist(const uint32_t* __restri
 
 // One CTA per digit: exclusive scan of hist[d][0..nblocks) in place, total to
 // totals[d].
-__global__ void __launch_bounds__(1024) k_sort_scan(uint32_t* __restrict__ hist, uint32_t nblocks,
+__global__ void __launch_bounds__(1024) k_sort_scan(uint32_t* hist, uint32_t nblocks,
                                                      uint32_t* __restrict__ totals) {
   __shared__ uint32_t s_warp[32];
   __shared__ uint32_t s_carry;
@@ -119,12 +119,12 @@ __global__ void __launch_bounds__(1024) k_sort_scan(uint32_t* __restrict__ hist,
 }
 
 template <int ROUNDS>
-__global__ void __launch_bounds__(kThreads) k_sort_scatter(const uint32_t* __restrict__ keys_in,
-                                                      const uint32_t* __restrict__ vals_in, int iota,
+__global__ void __launch_bounds__(kThreads) k_sort_scatter(const uint32_t* keys_in,
+                                                      const uint32_t* vals_in, int iota,
                                                       uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
                                                       uint32_t n, int shift, uint32_t nblocks,
-                                                      const uint32_t* __restrict__ hist,
-                                                      const uint32_t* __restrict__ totals, int by_tile) {
+                                                      const uint32_t* hist,
+                                                      const uint32_t* totals, int by_tile) {
   __shared__ uint32_t s_base[kBins];           // global base of each digit for this tile
   __shared__ uint32_t s_cnt[kWarps][kBins];    // per-warp digit counts of the current round
   __shared__ uint32_t s_pre[kWarps][kBins];    // per-warp digit prefix of the current round
