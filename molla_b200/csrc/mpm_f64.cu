@@ -165,7 +165,9 @@ __device__ __forceinline__ void record64(const Scene64& sc, const State64& st, i
   const double m = st.mass[i];
 #pragma unroll
   for (int k = 0; k < 3; ++k) tau[k] = 2.0 * md.mu * h * (scl[k] - 1.0) * scl[k] + md.lam * h * (J - 1.0) * J;
-  const double k4 = -sc.dt * st.vol[i] * 4.0 * sc.inv_dx;
+  // 4/dx^2 S d with d = (i - fx) dx: inv_dx is the reference's 1/dx rounded to
+  // FP32, so that inv_dx dx is 1 to 6e-8 only (exactly for powers of two)
+  const double k4 = -sc.dt * st.vol[i] * 4.0 * sc.inv_dx * (sc.inv_dx * sc.dx);
   double Bd[9];
 #pragma unroll
   for (int c = 0; c < 3; ++c)
