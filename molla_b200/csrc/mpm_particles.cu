@@ -676,8 +676,10 @@ __global__ void __launch_bounds__(kGatherThreads, 5) k_g2p(PoolDev p, double tol
     }
     const SceneDev& sc = w.sc;
     uint32_t* status = p.status + (size_t)sc.status * kStatusWords;
-    // a latched fault, a spent substep budget or a retired scene: stand still
-    if (!scene_frozen(status) && sc.live) {
+    // A latched fault, a spent substep budget or a retired scene: stand still.  A
+    // vote, since another warp may latch a fault between two lanes' reads and
+    // all lanes must go the same way around the warp barriers below.
+    if (__all_sync(0xffffffffu, !scene_frozen(status) && sc.live)) {
       const uint32_t tw = sc.w;
       const uint32_t tx = unit.tile % tw, ty = (unit.tile / tw) % tw, tz = unit.tile / (tw * tw);
       const int rx = 4 * (int)tx - 1, ry = 4 * (int)ty - 1, rz = 4 * (int)tz - 1;
@@ -694,7 +696,7 @@ __global__ void __launch_bounds__(kGatherThreads, 5) k_g2p(PoolDev p, double tol
             tma_load_box(w.vel, p.vel_maps + unit.scene, 4 * rx, ry, rz, &w.bar);
           }
           const uint32_t parity = w.parity;
-          if (!mbar_wait_bounded(&w.bar, parity)) {
+          if (!__all_sync(0xffffffffu, mbar_wait_bounded(&w.bar, parity))) {
             // The copy did not arrive: report it, wait once more (bounded)
             // for it and stop this warp.
             if (lane == 0) atomicOr(status, kFaultDeviceWait);

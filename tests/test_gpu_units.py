@@ -87,3 +87,34 @@ def test_all_fp64_positions_off_the_grid(engine, n):
     assert np.abs(vel - st["vel"]).max() < 1e-7
     assert np.abs(F - st["F"]).max() < 1e-8
     sim.close()
+
+
+@pytest.mark.parametrize("value", [np.nan, 1.0e30])
+def test_faults_all_over_a_large_scene(engine, value):
+    """Particles with a bad F all over a scene of more than 65,536 particles, whose
+    gather runs by warps on their own: some latch the fault (not finite: in the
+    call's record pass; out of the SVD's range: in the gather) while others of the
+    same launch find it latched.  The call ends and the scene stands still."""
+    n = 100_000
+    cfg = config(48, n)
+    rng = np.random.default_rng(5)
+    sim = m.MpmSimulation.new(engine, cfg)
+    sim.set_particles(rng.uniform(0.2, 0.7, size=(n, 3)).astype(np.float32))
+    sim.step_n(1e-4, 2)
+    C0, F0, jp0 = sim.read_particle_state()
+    F = F0.copy()
+    F[rng.choice(n, 3000, replace=False), 4] = value
+    sim.write_particle_state(F=F)
+    sim.step_n(1e-4, 3)
+    s = sim.read_active_grid_status()
+    assert s.numerical_fault and s.completed_substeps <= 3
+    before = (sim.read_positions(), sim.read_velocities(), *sim.read_particle_state())
+    sim.step_n(1e-4, 3)
+    after = (sim.read_positions(), sim.read_velocities(), *sim.read_particle_state())
+    for a, b in zip(before, after):
+        assert np.array_equal(a, b, equal_nan=True)
+    sim.write_particle_state(C_=C0, F=F0, jp=jp0)
+    sim.reset_active_grid()
+    sim.step_n(1e-4, 3)
+    assert not sim.read_active_grid_status().faulted()
+    sim.close()
