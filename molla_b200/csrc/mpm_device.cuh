@@ -168,9 +168,10 @@ enum Work : int { kWorkGather32 = 0, kWorkGather64 = 1, kWorkScatter = 2, kWorkW
 // the one before them still runs (launch_next allows it as soon as every CTA
 // of the running kernel has started) and wait here for its results before
 // they touch anything it writes.
-// A kernel that waits takes its inputs without __restrict__: a load
-// through a const __restrict__ parameter counts as a read of memory that never
-// changes while the kernel runs, and may be moved above the wait.
+// A kernel that waits, and every function it calls, takes what the kernels before
+// it write without const __restrict__ and without __ldg: such a load counts as a
+// read of memory that nobody writes for the kernel's whole life, which begins
+// before its wait ends; it may be moved above the wait or served by a stale line.
 __device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -192,7 +193,7 @@ __device__ __forceinline__ uint32_t unit_slot(const PoolDev& p, uint32_t n32, ui
 // scene record, or a copy of its grid fields (n, w, key_off, tile_cap,
 // grid_off).
 template <class SC>
-__device__ __forceinline__ int64_t node_index(const SC& sc, const uint32_t* __restrict__ tile_slot, int ix,
+__device__ __forceinline__ int64_t node_index(const SC& sc, const uint32_t* tile_slot, int ix,
                                               int iy, int iz) {
   const int n = (int)sc.n;
   if ((unsigned)ix >= (unsigned)n || (unsigned)iy >= (unsigned)n || (unsigned)iz >= (unsigned)n) return -1;

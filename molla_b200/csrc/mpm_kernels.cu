@@ -503,8 +503,8 @@ __global__ void k_items(const uint32_t* __restrict__ sorted_keys, uint32_t n_liv
 // a warp the cells are in the order of their particle counts (thread c
 // counts cell c in the item's slot keys, sorted by cell within a tile, by
 // binary search).  The four cells with b of 30 or 31 go to the spare lanes.
-__device__ __forceinline__ void item_order_one(const Item* __restrict__ items, uint32_t it,
-                                               const uint32_t* __restrict__ slot_key, uint8_t* __restrict__ item_order,
+__device__ __forceinline__ void item_order_one(const Item* items, uint32_t it,
+                                               const uint32_t* slot_key, uint8_t* __restrict__ item_order,
                                                uint32_t (&s_cnt)[64], uint8_t (&s_pair)[32][2],
                                                uint32_t (&s_fill)[32]) {
   const Item item = items[it];

@@ -62,8 +62,8 @@ __device__ __forceinline__ uint32_t base_key(const SceneDev& sc, const int* base
 // reference's out-of-grid skip.  Kept out of line and rolled so that the
 // unrolled shared-memory path stays small; it takes scalars and writes
 // v (3) and G = sum w gv d^T (9) to out.
-__device__ __noinline__ void gather_global(const float4* __restrict__ vel_pool, const SceneDev& sc,
-                                           const uint32_t* __restrict__ tile_slot, float xp0, float xp1, float xp2,
+__device__ __noinline__ void gather_global(const float4* vel_pool, const SceneDev& sc,
+                                           const uint32_t* tile_slot, float xp0, float xp1, float xp2,
                                            float* out) {
   const float xp[3] = {xp0, xp1, xp2};
   const int win[3] = {sc.winx, sc.winy, sc.winz};
@@ -84,7 +84,7 @@ __device__ __noinline__ void gather_global(const float4* __restrict__ vel_pool, 
     const int i = q / 9, j = (q / 3) % 3, k = q % 3;
     const int64_t c = node_index(sc, tile_slot, base[0] + i, base[1] + j, base[2] + k);
     if (c < 0) continue;
-    const float4 g = __ldg(&vel_pool[c]);
+    const float4 g = vel_pool[c];
     const float wt = w[0][i] * w[1][j] * w[2][k];
     const float gv[3] = {wt * g.x, wt * g.y, wt * g.z};
     for (int r = 0; r < 3; ++r) {
@@ -734,7 +734,7 @@ __global__ void __launch_bounds__(kGatherThreads, 5) k_g2p(PoolDev p, double tol
           for (uint32_t r = lane; r < (uint32_t)kRegionNodes; r += 32) {
             const int64_t c =
                 node_index(sc, p.tile_slot, rx + (int)(r & 7u), ry + (int)((r >> 3) & 7u), rz + (int)(r >> 6));
-            w.vel[r] = c >= 0 ? __ldg(&p.vel[c]) : make_float4(0.f, 0.f, 0.f, 0.f);
+            w.vel[r] = c >= 0 ? p.vel[c] : make_float4(0.f, 0.f, 0.f, 0.f);
           }
         }
       }
@@ -824,9 +824,9 @@ __global__ void __launch_bounds__(kGatherThreads, 5) k_g2p(PoolDev p, double tol
 // (256^3), from 0.239 to 0.222 ms at 4M and from 43.3 to 40 us at 500k (the
 // gather pays 0.03 ms for the form at 16M); swaps in flight together and a
 // warp for the margin cells, to 0.715 and 0.204 ms.
-__device__ __noinline__ void deposit_global(float4 c0, float4 c1, float4 c2, float4 c3, float4* __restrict__ acc,
-                                            uint8_t* __restrict__ touched, const SceneDev* __restrict__ scp,
-                                            const uint32_t* __restrict__ tile_slot) {
+__device__ __noinline__ void deposit_global(float4 c0, float4 c1, float4 c2, float4 c3, float4* acc,
+                                            uint8_t* touched, const SceneDev* scp,
+                                            const uint32_t* tile_slot) {
   const SceneDev& sc = *scp;
   const int win[3] = {sc.winx, sc.winy, sc.winz};
   const float Bd[9] = {c1.x, c1.y, c1.z, c1.w, c2.x, c2.y, c2.z, c2.w, c3.x};
@@ -955,7 +955,7 @@ __device__ __forceinline__ void bin_item(const float4* stage, const ScatterItem&
 // instead of eight, and the lanes that read the same record are served by one
 // broadcast); the two spare lanes of each warp (12 in all) take the 3 slabs of
 // slots 60..63.
-__device__ __forceinline__ uint32_t core_share(const uint8_t* __restrict__ order) {
+__device__ __forceinline__ uint32_t core_share(const uint8_t* order) {
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t q = warp * 2u + (lane - 30u);  // spare-lane index when lane >= 30
   const uint32_t slot = lane < 30u ? warp * 10u + lane / 3u : 60u + q / 3u;
@@ -1236,7 +1236,7 @@ __global__ void __launch_bounds__(kFusedThreads, 2) k_g2p2g(PoolDev p, double to
     for (int r = threadIdx.x; r < kRegionNodes; r += kFusedThreads) {
       const int64_t c = node_index(s_sc, p.tile_slot, s_item.rx + (r & 7), s_item.ry + ((r >> 3) & 7),
                                    s_item.rz + (r >> 6));
-      s_vel[r] = c >= 0 ? __ldg(&p.vel[c]) : make_float4(0.f, 0.f, 0.f, 0.f);
+      s_vel[r] = c >= 0 ? p.vel[c] : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     const uint32_t share = threadIdx.x < 192 ? core_share(p.item_order + (size_t)slot * 64) : 0u;
     __syncthreads();
@@ -1285,7 +1285,7 @@ __global__ void __launch_bounds__(kDetThreads, 2) k_p2g_det(PoolDev p, float4* _
   for (uint32_t it = blockIdx.x; it < n_items; it += gridDim.x) {
     const uint32_t slot = item_slot(p, n32, it);
     const Item item = p.items[slot];
-    const SceneDev* __restrict__ scp = p.scenes + item.scene;
+    const SceneDev* scp = p.scenes + item.scene;
     const uint32_t w = scp->w;
     const float ox = scp->ox, oy = scp->oy, oz = scp->oz, inv_dx = scp->inv_dx, dx = scp->dx;
     const int winx = scp->winx, winy = scp->winy, winz = scp->winz;
@@ -1316,10 +1316,10 @@ __global__ void __launch_bounds__(kDetThreads, 2) k_p2g_det(PoolDev p, float4* _
       float4 n0, n1, n2, n3;  // the next record, loaded while this one is added
       auto load = [&](uint32_t at) {
         const float4* r = rec + 4 * (size_t)at;
-        n0 = __ldg(r);
-        n1 = __ldg(r + 1);
-        n2 = __ldg(r + 2);
-        n3 = __ldg(r + 3);
+        n0 = r[0];
+        n1 = r[1];
+        n2 = r[2];
+        n3 = r[3];
       };
       if (s < end) load(s);
       for (; s < end; ++s) {
@@ -1421,7 +1421,7 @@ __global__ void k_combine_det(PoolDev p, const float4* blocks, const uint32_t* t
   for (uint32_t li = blockIdx.x; li < total; li += gridDim.x) {
     const uint32_t it = item_slot(p, n32, li);  // the item's slot, as tile_item holds it
     const Item item = p.items[it];
-    const SceneDev* __restrict__ scp = p.scenes + item.scene;
+    const SceneDev* scp = p.scenes + item.scene;
     const int w = (int)scp->w, n = (int)scp->n;
     const uint32_t key_off = scp->key_off;
     const int tx = (int)(item.tile % (uint32_t)w), ty = (int)((item.tile / (uint32_t)w) % (uint32_t)w),
