@@ -302,7 +302,6 @@ void Group::invalidate_graphs() {
   for (auto& kv : graphs)
     if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
   graphs.clear();
-  graph_seen.clear();
   ++epoch;
 }
 
@@ -1219,21 +1218,6 @@ void Group::step_graph(uint32_t substeps, uint32_t repeat, cudaStream_t st, cuda
     auto it = graphs.find(key);
     Graph g;
     if (it == graphs.end() || it->second.epoch != epoch) {
-      // A sequence is captured the second time it is asked for in a layout:
-      // capturing and instantiating one costs several times its launches (20
-      // substeps: about 2 ms against 0.3), and a served tick after an
-      // admission or a retirement is often never seen again.
-      cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-      MPM_CK(cudaStreamIsCapturing(st, &capture));
-      uint64_t& seen = graph_seen[key];
-      if (seen != epoch && capture == cudaStreamCaptureStatusNone) {
-        seen = epoch;
-        if (ev_begin && r == 0) MPM_CK(cudaEventRecord(ev_begin, st));
-        run_substeps(substeps, st);
-        if (ev_end && r + 1 == repeat) MPM_CK(cudaEventRecord(ev_end, st));
-        finish_retirements();
-        continue;
-      }
       const auto t_build0 = std::chrono::steady_clock::now();
       const uint64_t saved = eng->launches;
       cudaGraph_t graph = nullptr;

@@ -306,7 +306,6 @@ class Group {
     }
   };
   std::map<GraphKey, Graph> graphs;
-  std::map<GraphKey, uint64_t> graph_seen;  // epoch in which a sequence was first run (without a graph)
 
   // tile_cap > 0: sparse grid storage of that many 4^3-node tiles
   // (MpmSimulation::new_sparse, mpm.rs:846-853) instead of the dense n^3 grid.

@@ -446,3 +446,39 @@ def test_shapes_do_not_change_results(engine, shape):
     for sid, s in zip(ids, ss):
         assert np.abs(g.read_positions(sid) - alone(engine, s, 24)).max() < TOL
     g.close()
+
+
+def test_group_graphs_are_captured_and_replayed(engine):
+    """step_graph launches graphs from its first call on (stages are profiled in
+    plain launches alone, so the profile stays empty), and the sequences of a steady
+    loop (10 substeps, regrouped every 10) come back and are replayed; both match
+    plain steps.  A served tick builds its graph when it first runs."""
+    ss = small_scenes()[:3]
+    total = sum(s.n for s in ss)
+    cells = sum(s.grid_size ** 3 for s in ss) + 1024
+    a = m.MpmGroup(engine, 8, total, cells)
+    b = m.MpmGroup(engine, 8, total, cells)
+    ia = [a.add_scene(m.config_for_scene(s), s.rows, s.positions, s.ids, s.dt) for s in ss]
+    ib = [b.add_scene(m.config_for_scene(s), s.rows, s.positions, s.ids, s.dt) for s in ss]
+    for g in (a, b):
+        g.tune(sort_interval=10)
+    engine.profile(True)
+    try:
+        engine.reset_profile()
+        b.step_graph(10, 1)
+        assert sum(n for n, _ in engine.read_profile().values()) == 0
+        b.step_graph(10, 11)
+        assert sum(n for n, _ in engine.read_profile().values()) == 0
+    finally:
+        engine.profile(False)
+        engine.reset_profile()
+    for _ in range(12):
+        a.step(10)
+    for x, y in zip(ia, ib):
+        assert b.read_status(y).completed_substeps == 120
+        assert np.abs(a.read_positions(x) - b.read_positions(y)).max() < TOL
+    srv = m.MpmServer(engine, hbm_budget_bytes=64 << 20, max_scenes=8)
+    srv.submit(m.config_for_scene(ss[0]), ss[0].rows, ss[0].positions, ss[0].ids, ss[0].dt, 40)
+    srv.run(1, substeps_per_tick=20)
+    assert srv.stats()["graph_builds"] == 1
+    srv.close()
