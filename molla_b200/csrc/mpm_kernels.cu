@@ -282,11 +282,12 @@ __global__ void __launch_bounds__(kCellThreads) k_grid_jacobi(PoolDev p, const u
   const SceneDev& sc = p.scenes[sid];
   const uint64_t local64 = g - sc.grid_off;
   const uint32_t n = sc.n;
-  if (local64 >= (uint64_t)n * n * n) return;
   const float4 cur = src[g];
   const float m = p.acc[acc_in][g].x;
-  // massless, rigid-stamped (negative w) or done: copy through
-  if (sweep >= sc.jacobi_iters || m <= 1.0e-9f || !(m == m) || cur.w < 0.f) {
+  // Copy through: massless, rigid-stamped (negative w), the scene's sweeps done
+  // or none asked for (an explicit scene beside an implicit one; its storage may be
+  // sparse, with more nodes in its slots than n^3), or behind the grid.
+  if (sweep >= sc.jacobi_iters || m <= 1.0e-9f || !(m == m) || cur.w < 0.f || local64 >= (uint64_t)n * n * n) {
     dst[g] = cur;
     return;
   }

@@ -109,3 +109,30 @@ def test_group_mixes_sparse_and_dense_scenes(engine):
         assert np.abs(g.read_positions(sid) - pos).max() < TOL, sid
         assert not g.read_status(sid).faulted()
     g.close()
+
+
+@pytest.mark.parametrize("sweeps", [1, 2, 3])
+def test_sparse_explicit_scene_beside_an_implicit_one(engine, sweeps):
+    """A nearly full sparse scene whose slots hold more nodes than n^3 (34 nodes an
+    axis in 9^3 tiles of 64) moves beside a dense scene with Jacobi sweeps, which the
+    whole group's velocities pass through, as it does alone."""
+    n, grid = 20_000, 34
+    pts = np.random.default_rng(2).uniform(2.0 / grid, 31.0 / grid, size=(n, 3)).astype(np.float32)
+    kw = dict(grid_size=grid, cell_size=1.0 / grid, grid_origin=(0.0, 0.0, 0.0), gravity_y=-500.0, youngs=1.0e4, poisson=0.2,
+              friction_angle=0.0, boundary_friction=0.2, particle_mass=2.0e-3, particle_volume=1.0e-6, max_particles=n,
+              rheology=m.MpmRheology.Snow())
+    explicit = m.MpmConfig(**kw)
+    implicit = m.MpmConfig(**kw, time_step=m.MpmTimeStep.IMPLICIT, jacobi_iters=sweeps)
+    out = []
+    for beside in (False, True):
+        g = m.MpmGroup(engine, 4, 2 * n, 64 * 729 + grid ** 3 + 1024)
+        sid = g.add_scene(explicit, [explicit.rheology], pts, np.zeros(n, np.uint32), 1e-4, tile_capacity=729)
+        if beside:
+            g.add_scene(implicit, [implicit.rheology], pts, np.zeros(n, np.uint32), 1e-4)
+        g.step(10)
+        st = g.read_status(sid)
+        assert not st.faulted()
+        out.append(g.read_positions(sid))
+        g.close()
+    assert np.abs(out[0] - pts).max() > 1e-4
+    assert np.abs(out[0] - out[1]).max() < TOL
