@@ -1762,6 +1762,9 @@ int mpm_sim64_set_particles(mpm_sim64* sim, const double* xyz, uint32_t n) {
     MPM_CK(cudaMemcpyAsync(sim->F.ptr, F.data(), F.size() * 8, cudaMemcpyHostToDevice, st));
     MPM_CK(cudaMemcpyAsync(sim->mass.ptr, mass.data(), m * 8, cudaMemcpyHostToDevice, st));
     MPM_CK(cudaMemcpyAsync(sim->vol.ptr, vol.data(), m * 8, cudaMemcpyHostToDevice, st));
+    // k64_grid leaves the nodes that nothing is deposited to as they are: a
+    // faulted run before this one may have left them not finite
+    MPM_CK(cudaMemsetAsync(sim->gvel.ptr, 0, sim->gvel.bytes(), st));
     MPM_CK(cudaMemsetAsync(sim->status.ptr, 0, 16, st));
     MPM_CK(cudaStreamSynchronize(st));
   });

@@ -300,8 +300,10 @@ __global__ void __launch_bounds__(256) k64_grid(Scene64 sc, State64 st, int par,
     st.n_cells[par ^ 1] = 0u;
   }
   const double4 a = st.acc[c];
-  // a node nothing was deposited to is read by no particle with a weight
-  // other than zero; its old velocity is finite
+  // A node nothing was deposited to is read by no particle with a weight other
+  // than zero, and its old velocity is finite: set_particles clears it, and a
+  // velocity that is not finite faults the particle that deposited there in the
+  // same substep, after which nothing moves.
   if (a.x == 0.0 && a.y == 0.0 && a.z == 0.0 && a.w == 0.0) return;
   if (!last) st.acc[c] = make_double4(0.0, 0.0, 0.0, 0.0);
   const double m = a.x;

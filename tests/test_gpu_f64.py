@@ -50,3 +50,22 @@ def test_all_fp64_matches_oracle_on_any_cell_size(engine, grid, rheology):
     assert np.abs(st["F"] - np.eye(3).reshape(-1)).max() > 1e-4  # the stress acts
     assert np.abs(vel - st["vel"]).max() < 1e-11 * np.abs(st["vel"]).max()
     assert np.abs(pos - st["pos"]).max() < 1e-12
+
+
+def test_new_particles_after_a_fault_see_no_old_velocity(engine):
+    """A call whose gravity times dt overflows leaves infinite grid velocities and
+    faults; a new particle half-way between nodes has a stencil node of weight zero
+    that nothing is deposited to, with such a velocity on it."""
+    cfg = config(32, m.MpmRheology.Viscous(), 4096)
+    sim = m.MpmSimulation64(engine, cfg)
+    sim.set_particles(np.random.default_rng(0).uniform(0.25, 0.5, size=(4096, 3)))
+    sim.step_n(1.7e308, 1)
+    assert sim.read_active_grid_status().numerical_fault
+    x = np.array([[10.5 / 32, 12.5 / 32, 11.5 / 32]])
+    sim.set_particles(x)
+    sim.step_n(1e-4, 1)
+    assert not sim.read_active_grid_status().numerical_fault
+    pos, vel, _ = sim.read_state()
+    gy = float(np.float32(-9.8))
+    assert np.abs(vel - [[0.0, gy * 1e-4, 0.0]]).max() < 1e-15 and np.abs(pos - x - vel * 1e-4).max() < 1e-15
+    sim.close()
