@@ -349,7 +349,8 @@ template <class T> struct SvdOut {
 // rescaled by an exact power of two (2^200 or 2^-200) and the result by its
 // square root; this covers 1e-97 < x < 1e97 and costs a multiply, where a
 // fallback to IEEE double division and square root made the gather 3%
-// slower even untaken.  Infinite or NaN x gives NaN.
+// slower even untaken.  A finite x beyond 1e97 gives 0 (F of FP32 squares to
+// 1e78), an infinite or NaN x NaN.
 __device__ __forceinline__ double nr_rsqrt(double x) {
   double post = 1.0;
   if (!((float)x > 1.0e-37f && (float)x < 1.0e37f)) {

@@ -61,7 +61,15 @@ __device__ __forceinline__ void rot64(double (&a)[3][3], double* v, double tol, 
   const double apq = a[P][Q];
   max_off = fmax(max_off, fabs(apq));
   if (fabs(apq) < tol) return;
-  const double d = a[Q][Q] - a[P][P], e = 2.0 * apq;
+  double d = a[Q][Q] - a[P][P], e = 2.0 * apq;
+  // t takes d and e to a common factor: a power of two keeps the squares of a
+  // blown-up F's inside nr_rsqrt's range (an infinite one leaves a NaN)
+  const double m = fmax(fabs(d), fabs(e));
+  if (m > 1.0e40) {
+    const double k = scalbn(1.0, -ilogb(m));
+    d *= k;
+    e *= k;
+  }
   const double r2 = d * d + e * e;
   const double ri = nr_rsqrt(fabs(d) + r2 * nr_rsqrt(r2));
   const double t = (d >= 0.0 ? e : -e) * (ri * ri);
@@ -107,8 +115,12 @@ __device__ __forceinline__ void svd_ref64(const double* f, double* u, double* s,
     for (int r = 0; r < 3; ++r) m[r] = f[r] * v[3 * i] + f[3 + r] * v[3 * i + 1] + f[6 + r] * v[3 * i + 2];
     const double q = m[0] * m[0] + m[1] * m[1] + m[2] * m[2];
     const bool zero = q <= 1.0e-24;  // a NaN takes the other branch and reaches s
-    const double ri = zero ? 0.0 : nr_rsqrt(q);
+    double ri = zero ? 0.0 : nr_rsqrt(q);
     s[i] = q * ri;
+    if (q > 1.0e96) {  // beyond nr_rsqrt; an overflow reaches s
+      s[i] = sqrt(q);
+      ri = 1.0 / s[i];
+    }
 #pragma unroll
     for (int r = 0; r < 3; ++r) u[3 * i + r] = zero ? (i == r ? 1.0 : 0.0) : m[r] * ri;
   }

@@ -69,3 +69,34 @@ def test_new_particles_after_a_fault_see_no_old_velocity(engine):
     gy = float(np.float32(-9.8))
     assert np.abs(vel - [[0.0, gy * 1e-4, 0.0]]).max() < 1e-15 and np.abs(pos - x - vel * 1e-4).max() < 1e-15
     sim.close()
+
+
+@pytest.mark.parametrize("dt", [1e-4, 1e14, 1e26, 1e30])
+def test_blown_up_deformation_is_clamped(engine, dt):
+    """One substep of a huge dt deforms the particles whose stencil reaches the floor
+    by -g dt^2 / dx along y (1e30, 1e54, 1e62): that value comes out at its clamp, 20,
+    as the oracle's does (the other directions are rounding noise there).  1e-4
+    reaches no clamp and is compared whole."""
+    n = 4096
+    dt = float(np.float32(dt))
+    cfg = config(32, m.MpmRheology.Viscous(), n)
+    lo, hi = [0.3, 2.0 / 32, 0.3], [0.6, 0.2, 0.6]
+    pts = np.random.default_rng(3).uniform(lo, hi, size=(n, 3)).astype(np.float32).astype(np.float64)
+    (_, _, F), faulted, st = run_both(engine, cfg, pts, 1, dt=dt)
+    assert not faulted
+    if dt < 1.0:
+        assert np.abs(F - st["F"]).max() < 1e-12
+        return
+    floor = pts[:, 1] < 2.49 / 32
+    for f in (F, st["F"]):
+        assert np.abs(np.asarray(f)[floor, 4] + 20.0).max() < 1e-6
+
+
+def test_overflowing_deformation_faults(engine):
+    """F of 1e182, whose F^T F is not finite, faults."""
+    cfg = config(32, m.MpmRheology.Viscous(), 64)
+    sim = m.MpmSimulation64(engine, cfg)
+    sim.set_particles(np.random.default_rng(4).uniform([0.3, 2.0 / 32, 0.3], [0.4, 0.1, 0.4], size=(64, 3)))
+    sim.step_n(1e90, 1)
+    assert sim.read_active_grid_status().numerical_fault
+    sim.close()
