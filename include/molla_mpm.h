@@ -507,10 +507,10 @@ MPM_API int mpm_blake3(const void* data, size_t len, uint8_t* out32);
  * No reference counterpart as an API: it runs the reference substep
  * (reset, p2g, grid_update, g2p, plasticity; mpm.rs:2476-2551) with FP64
  * particle state, FP64 grid and the FP64 Jacobi SVD (tol 1e-14, 30 sweeps),
- * one GPU thread per particle or node.  It exists to measure the error of
- * the FP32 and FP32 + FP64-SVD modes against an all-FP64 run on the same
- * device; it is not tuned.  Explicit time step only; no groups, graphs or
- * ordering. */
+ * particle records and per-cell lists in place of the reference's scatter.
+ * It exists to measure the error of the FP32 and FP32 + FP64-SVD modes
+ * against an all-FP64 run on the same device.  Explicit time step only; no
+ * groups, graphs or ordering. */
 typedef struct mpm_sim64 mpm_sim64;
 MPM_API int mpm_sim64_create(mpm_engine* engine, const mpm_config* cfg, mpm_sim64** out);
 MPM_API int mpm_sim64_destroy(mpm_sim64* sim);

@@ -588,10 +588,11 @@ __device__ __forceinline__ void quad_weights(float fx, float* w) {
 // us), and no cancellation in Fc - R.  The FP64 form takes sc_i - 1 and J - 1 in
 // FP64, so that small strains keep their relative precision.
 //
-// FIXED (the fixed-order mode): B, with the stress as the reference writes it,
-// so that runs recorded by any earlier build replay bit for bit; otherwise B dx,
-// the change of a node's momentum from one node to the next along each axis (the
-// record's form).
+// FIXED (the fixed-order mode): B, with the stress as the reference writes it, so
+// that on cell sizes that are powers of two runs replay bit for bit what builds
+// before the deposit form computed (on others those builds let (x - o) / dx be
+// contracted, see lattice_pos); otherwise B dx, the change of a node's momentum
+// from one node to the next along each axis (the record's form).
 template <bool FIXED, class T>
 __device__ __forceinline__ void p2g_affine(const SvdOut<T>& svd, const MatDev& md, float jp, float mass, float vol,
                                            const float* C, float dt, float dx, float inv_dx, float* B) {

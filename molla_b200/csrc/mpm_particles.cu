@@ -206,8 +206,6 @@ struct NoRefill {
 };
 // Lattice x of a record that deposits nothing: outside every grid.
 constexpr float kOffGrid = 1.0e30f;
-static_assert(PY == PX + 1 && PZ == PX + 2 && MASS == F0 + 9 && VOL == F0 + 10 && JP == F0 + 11,
-              "the staged planes are two runs of consecutive planes");
 
 // The uniform values of the unit a gather warp is on, kept in shared memory so
 // that they hold no registers through the particle computation: the scene's
@@ -1191,7 +1189,8 @@ __global__ void __launch_bounds__(kScatterThreads, 4) k_p2g(PoolDev p, const __g
 // particles (the regrouping cuts them), so the records fit the stage; an
 // item that does not fit latches kFaultDeviceWait and is skipped.
 //
-// A fault latched before an item starts freezes the item (no gather, no
+// A fault latched when a CTA comes to a scene (its state is read with the
+// scene's first item in that CTA) freezes the CTA's items of it (no gather, no
 // deposit); a particle that faults during the gather deposits nothing (m = 0
 // in its record).  The scene is frozen from the next substep on.
 template <bool WRITE_KEYS, class SR>
