@@ -739,7 +739,7 @@ def measure_batched(args, quiet=False):
     shapes, tune = g.autotune_shapes(probe_substeps=32)
     chosen = shapes["sort_interval"]
     g.step_graph(max(3, args.batched_advance - args.batched_advance // 2), 1)
-    g.step_graph(steps, 1)  # captures the timed sequence's graph
+    g.step_graph(steps, 1)  # one more untimed call (the timed one's graph may be another: the regroup cadence is part of it)
     engine.synchronize()
     launches0 = engine.launch_count
     with ClockSampler(0) as clocks:

@@ -575,8 +575,8 @@ typedef struct mpm_server_stats {
   uint64_t faulted;
   /* tick graphs captured (a new tick shape, or a layout change since the
    * graph was made) and the host milliseconds spent capturing and
-   * instantiating or updating them; the tick latencies above time the
-   * graph launches alone */
+   * instantiating them; the tick latencies above time the graph launches
+   * alone */
   uint64_t graph_builds;
   double graph_build_ms;
 } mpm_server_stats;

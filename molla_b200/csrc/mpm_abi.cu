@@ -1476,8 +1476,8 @@ int mpm_server_run(mpm_server* server, uint32_t ticks, uint32_t substeps_per_tic
         if (server->queue.empty()) break;
         continue;
       }
-      // the tick's events bracket its graph launch alone: a capture or
-      // update of the graph before it is host time (graph_build_ms)
+      // the tick's events bracket its graph launch alone: a capture of the
+      // graph before it is host time (graph_build_ms)
       g.step_graph(len, 1, st, *server->e0, *server->e1);
       // The tick runs on the GPU while the caller goes on (submitting
       // requests); the next run, poll or stats call completes it.

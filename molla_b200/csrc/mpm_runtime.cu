@@ -302,7 +302,6 @@ void Group::invalidate_graphs() {
   for (auto& kv : graphs)
     if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
   graphs.clear();
-  ++epoch;
 }
 
 PoolDev Group::pool() const {
@@ -1217,7 +1216,7 @@ void Group::step_graph(uint32_t substeps, uint32_t repeat, cudaStream_t st, cuda
     const uint64_t regroups0 = regroups;
     auto it = graphs.find(key);
     Graph g;
-    if (it == graphs.end() || it->second.epoch != epoch) {
+    if (it == graphs.end()) {
       const auto t_build0 = std::chrono::steady_clock::now();
       const uint64_t saved = eng->launches;
       cudaGraph_t graph = nullptr;
@@ -1235,31 +1234,12 @@ void Group::step_graph(uint32_t substeps, uint32_t repeat, cudaStream_t st, cuda
       MPM_CK(cudaStreamEndCapture(st, &graph));
       g.kernels = eng->launches - saved;
       eng->launches = saved;
-      // A layout change (a scene added or retired, a regrouping moved)
-      // mostly changes launch parameters, not the sequence: update the
-      // existing executable graph in place when the topology allows, which
-      // costs far less host time than instantiating a new one.
-      bool updated = false;
-      if (it != graphs.end() && it->second.exec) {
-        cudaGraphExecUpdateResultInfo info{};
-        if (cudaGraphExecUpdate(it->second.exec, graph, &info) == cudaSuccess) {
-          g.exec = it->second.exec;
-          updated = true;
-        } else {
-          (void)cudaGetLastError();  // the failed update is not a sticky error
-          cudaGraphExecDestroy(it->second.exec);
-          it->second.exec = nullptr;
-        }
-      }
-      if (!updated) {
-        const cudaError_t ie = cudaGraphInstantiate(&g.exec, graph, 0);
-        if (ie != cudaSuccess) {
-          cudaGraphDestroy(graph);
-          MPM_CK(ie);
-        }
+      const cudaError_t ie = cudaGraphInstantiate(&g.exec, graph, 0);
+      if (ie != cudaSuccess) {
+        cudaGraphDestroy(graph);
+        MPM_CK(ie);
       }
       cudaGraphDestroy(graph);
-      g.epoch = epoch;
       // run_substeps advanced the host bookkeeping; rewind it, the launch
       // below applies the same transition.
       cur = cur0;

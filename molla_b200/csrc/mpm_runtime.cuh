@@ -288,13 +288,11 @@ class Group {
   // at most kStageMax, the scatter's shared-memory record stage.
   uint32_t item_chunk = kStageMax;
   uint64_t substeps_done = 0;
-  uint64_t epoch = 1;  // bumps on every change that invalidates captured graphs
 
   // graph cache: key -> instantiated graph + its kernel count
   struct Graph {
     cudaGraphExec_t exec = nullptr;
     uint64_t kernels = 0;
-    uint64_t epoch = 0;
   };
   struct GraphKey {
     uint32_t substeps, since, interval, flags;
