@@ -46,10 +46,13 @@ def test_item_sizes_match_oracle_grid(engine, n):
     sim.close()
 
 
+@pytest.mark.parametrize("fused", ["0", "1"])
 @pytest.mark.parametrize("speed", [2.0, 40.0])
-def test_moved_particles_still_deposit(engine, speed):
+def test_moved_particles_still_deposit(engine, speed, fused, monkeypatch):
     """Without a regrouping for 20 substeps particles end up in margin cells
-    (2 m/s: 0.6 cells) or outside their tile's block (40 m/s: 13 cells)."""
+    (2 m/s: 0.6 cells) or outside their tile's block (40 m/s: 13 cells); deposited
+    by the separate scatter and by the fused kernel."""
+    monkeypatch.setenv("MOLLA_MPM_FUSED", fused)
     cfg = config(64, 20_000)
     cfg.gravity_y = 0.0
     rng = np.random.default_rng(3)

@@ -1,8 +1,8 @@
-"""The gather's units and the grid update's block lists at their edges: particle
-counts around one and two rounds of a warp and the sizes at which the unit
-changes, grids below, at and off the 8^3 velocity box, against the oracle; sparse
-storage whose particles leave the block of their tile; and the fixed-order mode
-against itself.
+"""The gather's units and the grid update's block lists at their edges: tiles of
+particle counts around the rounds of a warp and the ends of units, at each unit
+size the group's particle count picks; grids below, at and off the 8^3 velocity
+box, against the oracle; sparse storage whose particles leave the block of their
+tile; and faults all over a scene.
 
 Tolerances: one substep in FP32, |dx| <= 1e-6 and |dv| <= 1e-5 max(1, |v|) (see
 test_gpu_parity)."""
@@ -41,6 +41,37 @@ def test_units_match_oracle(engine, grid, n, svd):
     v = sim.read_velocities()
     assert (np.abs(v - st["vel"]) / np.maximum(np.abs(st["vel"]), 1.0)).max() <= 1e-5
     sim.close()
+
+
+@pytest.mark.parametrize("beside,unit", [(0, 32), (250_000, 64), (4_000_000, 128), (24_000_000, 640)])
+def test_unit_sizes_and_remainders(engine, beside, unit):
+    """One substep of tiles of 1 to 1,300 particles, in units of each size: the
+    unit grows with the group's particles (64 from 189,441 on, a twelfth of the
+    particles per resident warp above, at most 640), so a scene beside sets it."""
+    counts = [1, 31, 32, 33, 63, 64, 65, 95, 96, 97, 127, 128, 129, 160, 639, 640, 641, 673, 1281, 1300]
+    grid, dt = 64, 1e-3
+    rng = np.random.default_rng(unit)
+    pts = []
+    for k, c in enumerate(counts):  # base cells of every other tile: nothing is shared
+        tile = np.array([2 + 2 * (k % 5), 2 + 2 * (k // 5), 6])
+        pts.append((4 * tile + 0.51 + 3.97 * rng.random((c, 3))) / grid)
+    pts = np.concatenate(pts).astype(np.float32)[rng.permutation(sum(counts))]
+    cfg = config(grid, len(pts))
+    cfg.gravity_y = -500.0
+    g = m.MpmGroup(engine, 2, len(pts) + beside, grid ** 3 + 256 ** 3 + 1024)
+    sid = g.add_scene(cfg, [cfg.rheology], pts, np.zeros(len(pts), np.uint32), dt)
+    if beside:
+        other = config(256, beside)
+        g.add_scene(other, [other.rheology], rng.random((beside, 3), np.float32) * np.float32(0.8) + np.float32(0.1),
+                    np.zeros(beside, np.uint32), 1e-5)
+    g.step(1)
+    got = g.read_positions(sid)
+    assert not g.read_status(sid).faulted()
+    g.close()
+    st = O.init_state(pts, mass=cfg.particle_mass, volume=cfg.particle_volume)
+    O.step(O.make_scene(cfg, [cfg.rheology], dt), st, 1, precision="f32")
+    assert np.abs(st["pos"] - pts)[:, 1].min() > 4e-4  # every particle falls
+    assert np.abs(got - st["pos"]).max() <= 1e-6
 
 
 @pytest.mark.parametrize("speed", [0.5, 30.0])
