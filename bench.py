@@ -57,11 +57,11 @@ KERNEL_BYTES = {
 }
 # DRAM bytes per particle per launch (dram__bytes_read.sum +
 # dram__bytes_write.sum) from one ncu capture of each kernel of the separate
-# substep on the medium workload (128^3 grid, 2M particles, substep ~250),
+# substep on the medium workload (128^3 grid, 2M particles, after about 150 substeps),
 # scaled by particle count.
 MEASURED_TRAFFIC_PER_PARTICLE = {
-    "GridToParticle": 156.4,
-    "ParticleToGrid": 70.9,
+    "GridToParticle": 155.2,
+    "ParticleToGrid": 69.6,
 }
 # The fused gather + scatter (k_g2p2g, groups of at most 64k particles)
 # keeps the 64-byte record in shared memory: 180 - 64 B per particle, and per
@@ -69,7 +69,7 @@ MEASURED_TRAFFIC_PER_PARTICLE = {
 FUSED_BYTES = (116, 32)
 # ncu DRAM bytes per particle of k_g2p2g on the 1M-particle scaled cube
 # (state 160 MB, just above L2).
-MEASURED_TRAFFIC_FUSED_PER_PARTICLE = 76.5
+MEASURED_TRAFFIC_FUSED_PER_PARTICLE = 75.9
 # Whole-step model of the survey (separate P2G and G2P passes):
 # 268 B per particle-step + 56 B per active cell-step.
 STEP_BYTES_PER_PARTICLE = 268

@@ -592,7 +592,7 @@ struct __align__(128) GatherWarp {
 // the list, its first by its index and each later one from the counter, with
 // the velocity block of the unit's tile fetched into its own shared memory by
 // one TMA box, and shares no barrier with the other warps of its CTA.
-// What bounds it: instruction issue (64% of the slots; 61 warp instructions a
+// What bounds it: instruction issue (65% of the slots; 58 warp instructions a
 // particle of mixed materials) and, behind that, the dependent chains of the
 // SVD and instruction fetch (41 KB of code; it was 55, of which a second SVD
 // for a case that never came was 13); 0.4 of the DRAM rate.  From a CTA per
@@ -816,7 +816,7 @@ __global__ void __launch_bounds__(kGatherThreads, 5) k_g2p(PoolDev p, double tol
 // a second bounded wait for its copy in flight.
 //
 // What bounds it: instruction issue and shared-memory latency, not bytes
-// (15% of DRAM rate).  Lists instead of a counting sort, records written in
+// (17% of DRAM rate).  Lists instead of a counting sort, records written in
 // deposit form by the gather instead of rewritten here, and the item's frame
 // in shared memory took it from 0.832 to 0.773 ms on a 16M-particle scene
 // (256^3), from 0.239 to 0.222 ms at 4M and from 43.3 to 40 us at 500k (the
